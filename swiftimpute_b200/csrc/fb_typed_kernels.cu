@@ -27,6 +27,8 @@
 #include "fb_typed.hpp"
 #include "philox.cuh"
 
+#include <type_traits>
+
 namespace si {
 namespace {
 
@@ -428,227 +430,303 @@ __device__ __forceinline__ void init_forward(float (&a)[LM], uint32_t em) {
     for (int k = 0; k < LM; ++k) a[k] = ((em >> k) & 1u) ? 1.f : 0.f;
 }
 
-constexpr uint32_t kChainBlock = 8;  // anchors per block of list entries
+// Steps per staged block: two blocks of a direction's records stay under 48 KB
+// of shared memory, five CTAs an SM.
+__host__ __device__ constexpr uint32_t chain_block(uint32_t LM) { return LM <= 8 ? 8u : 4u; }
+constexpr uint32_t kChainPrep = 2;                            // warps that prepare a chain warp's steps
+constexpr uint32_t kChainThreads = 32 * (1 + kChainPrep);
+constexpr uint32_t kChainAhead = 3;                           // blocks of list entries in flight before the one prepared
 
-// One chain per lane with all LM slots in registers: even warps run forward
-// chains, odd warps the backward chains of the same 32 samples. The warp
-// steps in lockstep to the longest of its chains (a finished chain holds its
-// state), in blocks of kChainBlock anchors. A block's list entries are loaded
-// two blocks ahead and its run-table entries one block ahead, so a step's
-// dependent path is its own arithmetic: the slot update, the sum over the
-// slots and the power-of-two rescale (and, backward, the unit's log when
-// beta's e^-999 floor matters). Checkpoints: backward vector and the log of
-// its unit at anchors k % C == 0 (window starts); forward vector at anchors
-// k % (K C) == 0.
+// What a chain's step needs beyond its state, per lane: the emission over the
+// slots as 0/1 factors, the run's {Q, S} and, backward, G(n) - 999 (the floor's
+// log before the unit) and the unit's change n log rho - 999 shift.
 template <int LM>
-__global__ void __launch_bounds__(32) anchor_chain_kernel(TypedArgs A) {
-    constexpr uint32_t KB = kChainBlock;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const bool forward = (wg & 1u) == 0;
-    const uint32_t s = (wg >> 1) * 32 + lane;
+struct ChainStage {
+    float4 mask[chain_block(LM)][LM / 4][32];
+    float2 qs[chain_block(LM)][32];
+    double g[chain_block(LM)][32];
+    double c[chain_block(LM)][32];
+};
+
+// One chain per lane with all LM slots in registers; a CTA runs the forward
+// (even blocks) or the backward (odd blocks) chains of a group of 32 samples,
+// warp 0 the recursion, all lanes at the same anchor in a step.
+// Bound: the dependent recursion, one warp's steps one after the other, so each
+// instruction of that warp counts and it must not wait for memory. The CTA's
+// other warps therefore prepare the steps: list entries come by cp.async blocks
+// ahead, a block's table entries together, and finished records stand in shared
+// memory (two blocks, one barrier a block). A step is then the masked slot
+// update (an emission bit is a factor 0 or 1, exact), the sum over the slots and
+// the power-of-two rescale and, backward, the unit's log and the floor, without
+// a branch.
+// A forward chain past its last anchor, and a backward chain before its first,
+// step over records that mean nothing: nothing of theirs is stored, and a
+// backward chain sets its state when its first anchor comes. Checkpoints:
+// backward vector and the log of its unit at anchors k % C == 0 (window
+// starts); forward vector at anchors k % (K C) == 0.
+// Measured against one warp that loaded, looked up and stepped by itself (launch,
+// CUDA events): 10,000 targets x 2,942 anchors, L = 8: 0.95 -> 0.59 ms; 2,003 x
+// 1,876: 0.58 -> 0.27; one target of 329: 0.101 -> 0.055; 4,000 x 1,000 at L = 16:
+// 0.39 -> 0.17; 1,500 x 601 at L = 32: 0.29 -> 0.19. A backward step alone takes
+// 215 cycles (most of it the floor: FP64 difference, conversion, expf), a forward
+// one 130. Not kept: one preparing warp (it set the pace: 0.96 ms), table entries
+// by cp.async one by one (the same), factors looked up by the chain warp at L >= 16
+// (0.19 and 0.22 ms), four preparing warps at L = 32 (0.20).
+template <int LM>
+__global__ void __launch_bounds__(kChainThreads, LM <= 16 ? 5 : 3) anchor_chain_kernel(TypedArgs A) {
+    constexpr uint32_t KB = chain_block(LM), H = LM / 2, Q4 = LM / 4;
+    __shared__ __align__(16) ChainStage<LM> stage[2];
+    __shared__ __align__(16) uint32_t rpos[kChainAhead + 2][KB][32], rem[kChainAhead + 2][KB][32];  // list entries
+    __shared__ float4 nibble[16];  // four emission bits as factors
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool forward = (blockIdx.x & 1u) == 0;
+    const uint32_t s = (blockIdx.x >> 1) * 32 + lane;
     const bool live = s < A.B;
-    // A lane past the batch's end takes the last sample's tables: its discarded
-    // lookups (gap 0) then read the tables like its warp's live lanes instead of
-    // evaluating the FP64 closed form past a table of zero entries every step.
+    // A lane past the batch's end takes the last sample's tables (gap 0 is in every
+    // table; past an empty table each lookup would evaluate the FP64 closed form).
     const View v = view_of(A, live ? s : A.B - 1);
     uint32_t NA = 0;
     unsigned long long base = 0, wb = 0;
     if (live) {
-        base = A.aoff[s >> 5] + lane;
+        base = A.aoff[s >> 5];
         wb = A.woff[s >> 5] + lane;
         NA = A.counts[s];
     }
     const uint32_t NAw = __reduce_max_sync(0xffffffffu, NA);
-    if (NAw == 0) return;  // whole warp
+    if (NAw == 0) return;  // every warp of the CTA
     const Tabs& tb = v.r.tabs;
-    const uint32_t* apos = A.apos + base;  // entry k at apos[32 k]
-    const uint32_t* aemk = A.aem + base;
-    auto pos = [&](uint32_t k) { return apos[32ull * k] & ~kShiftBit; };
-    auto aem = [&](uint32_t k) { return aemk[32ull * k]; };
-    const uint32_t C = A.C, K = A.K;
-    auto ck = [&](uint32_t w) { return wb + 32ull * w; };  // window w's checkpoint entry
-    constexpr uint32_t H = LM / 2;  // slot pairs
+    // Block b holds anchors [b KB, b KB + KB) of the group's lists. A forward chain steps
+    // over anchors 1, 2, ... in blocks 0, 1, ...; a backward chain over NAw - 2, ... , 0
+    // in blocks NB - 1, NB - 2, ... . Iteration i takes block blk(i).
+    const uint32_t NB = (NAw + KB - 1) / KB;
+    auto blk = [&](uint32_t i) { return forward ? i : NB - 1 - i; };
+    if (threadIdx.x < 16)
+        nibble[threadIdx.x] = make_float4(threadIdx.x & 1u ? 1.f : 0.f, threadIdx.x & 2u ? 1.f : 0.f,
+                                          threadIdx.x & 4u ? 1.f : 0.f, threadIdx.x & 8u ? 1.f : 0.f);
+
+    if (warp > 0) {
+        const uint32_t* apos = A.apos + __shfl_sync(0xffffffffu, base, 0);  // the group's lists
+        const uint32_t* aem = A.aem + __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t pt = threadIdx.x - 32;
+        // block of iteration i: KB x 128 contiguous bytes of positions and of emissions
+        auto fetch = [&](uint32_t i) {
+            if (i < NB) {
+                const uint32_t slot = i % (kChainAhead + 2), k0 = blk(i) * KB;
+                for (uint32_t x = pt; x < KB * 8; x += 32 * kChainPrep)
+                    if (k0 + x / 8 < NAw) {
+                        cp_async16(&rpos[slot][0][0] + 4 * x, apos + 32ull * k0 + 4 * x);
+                        cp_async16(&rem[slot][0][0] + 4 * x, aem + 32ull * k0 + 4 * x);
+                    }
+            }
+            cp_async_commit();
+        };
+        // records of iteration i; a record's run lies between its anchor and the one before
+        // it in list order (forward) or after it (backward), perhaps in a neighbour block
+        auto prepare = [&](uint32_t i) {
+            const uint32_t slot = i % (kChainAhead + 2), k0 = blk(i) * KB;
+            const uint32_t before = (i + kChainAhead + 1) % (kChainAhead + 2);  // slot of iteration i - 1
+            ChainStage<LM>& S = stage[i & 1u];
+            constexpr uint32_t JP = KB / kChainPrep;
+            uint32_t n[JP], nt[JP], em[JP], sh[JP];
+            float2 qs[JP];
+            double g[JP];
+            bool past = false;
+#pragma unroll
+            for (uint32_t jj = 0; jj < JP; ++jj) {
+                const uint32_t j = (warp - 1) * JP + jj, k = k0 + j;
+                const uint32_t pe = rpos[slot][j][lane];
+                uint32_t po;  // the neighbour's position
+                if (forward) po = j ? rpos[slot][j - 1][lane] : rpos[before][KB - 1][lane];
+                else po = j + 1 < KB ? rpos[slot][j + 1][lane] : rpos[before][0][lane];
+                const bool ok = forward ? (k >= 1 && k < NA) : k + 1 < NA;
+                n[jj] = ok ? (forward ? pe - po : po - pe) & ~kShiftBit : 0u;
+                sh[jj] = pe >> 31;
+                em[jj] = rem[slot][j][lane];
+                past |= n[jj] >= tb.NT;
+                nt[jj] = min(n[jj], tb.NT - 1);
+            }
+#pragma unroll
+            for (uint32_t jj = 0; jj < JP; ++jj) {  // the block's table entries in flight together
+                qs[jj] = __ldg(tb.QS + nt[jj]);
+                g[jj] = forward ? 0.0 : __ldg(tb.G + nt[jj]);
+            }
+            if (past) {  // runs longer than the tables
+#pragma unroll
+                for (uint32_t jj = 0; jj < JP; ++jj)
+                    if (n[jj] >= tb.NT) {
+                        qs[jj] = tabQS(tb, n[jj]);
+                        g[jj] = tabG(tb, n[jj]);
+                    }
+            }
+#pragma unroll
+            for (uint32_t jj = 0; jj < JP; ++jj) {
+                const uint32_t j = (warp - 1) * JP + jj;
+                S.qs[j][lane] = qs[jj];
+                if (!forward) {
+                    S.g[j][lane] = g[jj] - 999.0;
+                    S.c[j][lane] = fma(u2d(n[jj]), tb.lr, sh[jj] ? -999.0 : 0.0);
+                }
+#pragma unroll
+                for (uint32_t q = 0; q < Q4; ++q) S.mask[j][q][lane] = nibble[(em[jj] >> (4 * q)) & 15u];
+            }
+        };
+        for (uint32_t i = 0; i <= kChainAhead; ++i) fetch(i);
+        cp_async_wait_group<kChainAhead - 1>();  // the entries of iterations 0 and 1 have landed
+        __syncthreads();
+        prepare(0);
+        for (uint32_t i = 0; i < NB; ++i) {
+            cp_async_wait_group<kChainAhead - 1>();
+            __syncthreads();  // records i are ready, with the entries of i + 1; records i - 1 have been read
+            fetch(i + 1 + kChainAhead);  // into the slot of iteration i - 1
+            if (i + 1 < NB) prepare(i + 1);
+        }
+        return;
+    }
+
+    struct Rec {
+        float4 m[Q4];
+        float2 q;
+    };
+    auto read = [&](const ChainStage<LM>& S, uint32_t j) {
+        Rec r;
+        r.q = S.qs[j][lane];
+#pragma unroll
+        for (uint32_t i = 0; i < Q4; ++i) r.m[i] = S.mask[j][i][lane];
+        return r;
+    };
     auto store = [&](float* dst, const float2 (&x)[H]) {
 #pragma unroll
-        for (uint32_t q = 0; q < H / 2; ++q)
+        for (uint32_t q = 0; q < Q4; ++q)
             reinterpret_cast<float4*>(dst)[q] = make_float4(x[2 * q].x, x[2 * q].y, x[2 * q + 1].x, x[2 * q + 1].y);
     };
-    // a step's update of the slot pairs: em bit l ? g x_l + b : 0, its sum, and the power-of-two
-    // rescale that brings the sum into [1, 2) (the scale's exponent is -e)
-    auto update = [&](float2 (&x)[H], uint32_t em, float g, float b, float& sum, int& e) {
-        const float2 G2 = make_float2(g, g), B2 = make_float2(b, b);
-        float2 xn[H];
-#pragma unroll
-        for (uint32_t h = 0; h < H; ++h) {
-            const float2 t = __ffma2_rn(G2, x[h], B2);
-            xn[h] = make_float2(((em >> (2 * h)) & 1u) ? t.x : 0.f, ((em >> (2 * h + 1)) & 1u) ? t.y : 0.f);
-        }
+    // the sum of xn and the power-of-two rescale that brings it into [1, 2): x = xn 2^-e
+    auto rescale = [&](float2 (&x)[H], const float2 (&xn)[H], float& sum, int& bits) {
         const float s2 = vsum2<H>(xn);
-        const int bits = __float_as_int(s2) & 0x7f800000;
+        bits = __float_as_int(s2) & 0x7f800000;
         const float sc = __int_as_float(0x7f000000 - bits);
         const float2 S2 = make_float2(sc, sc);
 #pragma unroll
         for (uint32_t h = 0; h < H; ++h) x[h] = __fmul2_rn(xn[h], S2);
         sum = s2 * sc;
-        e = (bits >> 23) - 127;
     };
-    if (forward) {
-        // step k (anchor k = 1 .. NA - 1): the run from anchor k - 1, then anchor k's emission
-        float2 a[H];
-        uint32_t prev = 0;
+    // a step's update of the slot pairs: factor m_l (0 or 1) times (g x_l + b), summed and rescaled
+    auto update = [&](float2 (&x)[H], const float4 (&m)[Q4], float g, float b, float& sum, int& bits) {
+        const float2 G2 = make_float2(g, g), B2 = make_float2(b, b);
+        float2 xn[H];
 #pragma unroll
-        for (uint32_t h = 0; h < H; ++h) a[h] = make_float2(0.f, 0.f);
-        float sa = 0.f;
-        if (NA > 0) {
-            int e;
-            const uint32_t em = aem(0);
-#pragma unroll
-            for (uint32_t h = 0; h < H; ++h) a[h] = make_float2(1.f, 1.f);
-            update(a, em, 0.f, 1.f, sa, e);  // the emission of anchor 0 over uniform slots
-            prev = pos(0);
-            store(A.ckptF + ck(0) * LM, a);
+        for (uint32_t q = 0; q < Q4; ++q) {
+            const float2 m0 = make_float2(m[q].x, m[q].y), m1 = make_float2(m[q].z, m[q].w);
+            xn[2 * q] = __ffma2_rn(__fmul2_rn(G2, m0), x[2 * q], __fmul2_rn(B2, m0));
+            xn[2 * q + 1] = __ffma2_rn(__fmul2_rn(G2, m1), x[2 * q + 1], __fmul2_rn(B2, m1));
         }
-        uint32_t cc = C, ci = 1;  // anchors to the next checkpoint, its window
-        auto load = [&](uint32_t k0, uint32_t (&p)[KB], uint32_t (&e)[KB]) {
+        rescale(x, xn, sum, bits);
+    };
+    auto emission = [&](float2 (&xn)[H], uint32_t em) {
+#pragma unroll
+        for (uint32_t h = 0; h < H; ++h)
+            xn[h] = make_float2((em >> (2 * h)) & 1u ? 1.f : 0.f, (em >> (2 * h + 1)) & 1u ? 1.f : 0.f);
+    };
+    float2 x[H];
+    float sx = 0.f;
+    __syncthreads();
+    if (forward) {
+        // anchor 0's emission over uniform slots, then per anchor the run from the one before and its emission
+        const uint32_t KC = A.K * A.C;
+        float* ck = A.ckptF + wb * LM;  // the next checkpoint: every K-th window's entry
+        const size_t ckstep = (size_t)32 * A.K * LM;
+        float2 xn[H];
+        emission(xn, NA > 0 ? A.aem[base + lane] : 1u);
+        int bits;
+        rescale(x, xn, sx, bits);
+        if (NA > 0) store(ck, x);
+        uint32_t next = KC;  // its anchor
+        for (uint32_t i = 0; i < NB; ++i) {
+            __syncthreads();
+            const ChainStage<LM>& S = stage[i & 1u];
+            Rec r = read(S, 0);
 #pragma unroll
             for (uint32_t j = 0; j < KB; ++j) {
-                const uint32_t k = k0 + j;
-                p[j] = k < NA ? pos(k) : 0u;
-                e[j] = k < NA ? aem(k) : 0u;
-            }
-        };
-        auto tables = [&](uint32_t k0, const uint32_t (&p)[KB], uint32_t before, float2 (&q)[KB]) {
-#pragma unroll
-            for (uint32_t j = 0; j < KB; ++j) q[j] = tabQS(tb, k0 + j < NA ? p[j] - (j ? p[j - 1] : before) : 0u);
-        };
-        auto step = [&](uint32_t em, float2 q) {
-            int e;
-            update(a, em, q.x, sa * q.y, sa, e);
-            if (--cc == 0) {
-                if (ci % K == 0) store(A.ckptF + ck(ci) * LM, a);
-                ++ci;
-                cc = C;
-            }
-        };
-        uint32_t p0[KB], e0[KB], p1[KB], e1[KB];
-        float2 q0[KB];
-        load(1, p0, e0);
-        load(1 + KB, p1, e1);
-        tables(1, p0, prev, q0);
-        for (uint32_t k0 = 1; k0 < NAw; k0 += KB) {
-            uint32_t p2[KB], e2[KB];
-            float2 q1[KB];
-            load(k0 + 2 * KB, p2, e2);           // two blocks ahead
-            tables(k0 + KB, p1, p0[KB - 1], q1);  // one block ahead
-            if (__all_sync(0xffffffffu, k0 + KB <= NA)) {
-#pragma unroll
-                for (uint32_t j = 0; j < KB; ++j) step(e0[j], q0[j]);
-            } else {
-#pragma unroll
-                for (uint32_t j = 0; j < KB; ++j)
-                    if (k0 + j < NA) step(e0[j], q0[j]);  // a finished chain holds its state
-            }
-#pragma unroll
-            for (uint32_t j = 0; j < KB; ++j) {
-                p0[j] = p1[j]; e0[j] = e1[j]; q0[j] = q1[j];
-                p1[j] = p2[j]; e1[j] = e2[j];
+                Rec rn = r;
+                if (j + 1 < KB) rn = read(S, j + 1);
+                const uint32_t k = i * KB + j;
+                if (j || i) {  // anchor 0 is the start
+                    update(x, r.m, r.q.x, sx * r.q.y, sx, bits);
+                    if (k == next) {
+                        ck += ckstep;
+                        next += KC;
+                        if (k < NA) store(ck, x);
+                    }
+                }
+                r = rn;
             }
         }
     } else {
-        // step t handles anchor k = NA - 2 - t (t = 0 .. NA - 2): the run to anchor k + 1
-        float2 w[H];
-        uint32_t nextp = 0;
-        double logU = 0.0;
-#pragma unroll
-        for (uint32_t h = 0; h < H; ++h) w[h] = make_float2(0.f, 0.f);
-        float sw = 0.f;
+        const uint32_t C = A.C;
+        double logU = 0.0, logU0 = 0.0;
+        uint32_t em0 = 1u;
         if (NA > 0) {
-            const uint32_t pl = apos[32ull * (NA - 1)];
-            nextp = pl & ~kShiftBit;
-            logU = chain_end_logU(tb, v.len - 1 - nextp) - ((pl & kShiftBit) ? 999.0 : 0.0);
-            const uint32_t em = aem(NA - 1);
-#pragma unroll
-            for (uint32_t h = 0; h < H; ++h)
-                w[h] = make_float2(((em >> (2 * h)) & 1u) ? 1.f : 0.f, ((em >> (2 * h + 1)) & 1u) ? 1.f : 0.f);
-            sw = vsum2<H>(w);
-            if ((NA - 1) % C == 0) {
-                store(A.ckptB + ck((NA - 1) / C) * LM, w);
-                A.ckptU[ck((NA - 1) / C)] = logU;
-            }
+            const uint32_t pl = A.apos[base + lane + 32ull * (NA - 1)];
+            logU0 = chain_end_logU(tb, v.len - 1 - (pl & ~kShiftBit)) - ((pl & kShiftBit) ? 999.0 : 0.0);
+            em0 = A.aem[base + lane + 32ull * (NA - 1)];
         }
-        uint32_t cc = NA >= 2 ? (NA - 2) % C + 1 : 0u;  // anchors to the next checkpoint (k % C == 0)
-        uint32_t ci = NA >= 2 ? (NA - 2) / C : 0u;      // its window
-        auto load = [&](uint32_t t0, uint32_t (&p)[KB], uint32_t (&e)[KB], uint32_t (&h)[KB]) {
+        emission(x, em0);
+        sx = vsum2<H>(x);
+        uint32_t left = (NAw - 1) % C;  // anchors to the next checkpoint, a multiple of C
+        float* ckB = A.ckptB + (wb + 32ull * ((NAw - 1) / C)) * LM;  // its entries
+        double* ckU = A.ckptU + wb + 32ull * ((NAw - 1) / C);
+        const uint32_t first = __reduce_min_sync(0xffffffffu, NA);
+        for (uint32_t i = 0; i < NB; ++i) {
+            __syncthreads();
+            const ChainStage<LM>& S = stage[i & 1u];
+            const uint32_t k0 = (NB - 1 - i) * KB;
+            Rec r = read(S, KB - 1);
+            double g = S.g[KB - 1][lane], c = S.c[KB - 1][lane];
+            // kStart: a chain of the group starts in this block
+            auto steps = [&](auto kStart) {
 #pragma unroll
-            for (uint32_t j = 0; j < KB; ++j) {
-                const uint32_t t = t0 + j;
-                const bool ok = t + 2 <= NA;
-                const uint32_t k = NA - 2 - t;
-                const uint32_t pk = ok ? apos[32ull * k] : 0u;
-                p[j] = pk & ~kShiftBit;
-                e[j] = ok ? aem(k) : 0u;
-                h[j] = pk >> 31;
-            }
-        };
-        // per step: {Q, S} of the run, G(n) - 999 and the unit's change n log rho - 999 shift
-        auto tables = [&](uint32_t t0, const uint32_t (&p)[KB], const uint32_t (&h)[KB], uint32_t after,
-                          float2 (&q)[KB], double (&g)[KB], double (&c)[KB]) {
-#pragma unroll
-            for (uint32_t j = 0; j < KB; ++j) {
-                const uint32_t n = t0 + j + 2 <= NA ? (j ? p[j - 1] : after) - p[j] : 0u;
-                q[j] = tabQS(tb, n);
-                g[j] = tabG(tb, n) - 999.0;
-                c[j] = fma(u2d(n), tb.lr, h[j] ? -999.0 : 0.0);
-            }
-        };
-        auto step = [&](uint32_t em, float2 q, double g, double c) {
-            // the floor's log in units of U: fterm > 0, the floor dominates and the unit
-            // becomes U rho^n e^fterm; fterm <= -104, it is negligible (the common case:
-            // the carried terms alone, and the unit's bookkeeping stays off this step's path)
-            const double fterm = g - logU;
-            const bool big = fterm > 0.0;
-            float xs = 1.f, F = 0.f;
-            if (fterm > -104.0) {
-                const float ex = expf(-(float)fmin(fabs(fterm), 104.0));
-                xs = big ? ex : 1.f;  // scale of the carried terms
-                F = big ? 1.f : ex;   // the floor term
-            }
-            int e;
-            update(w, em, xs * q.x, fmaf(xs * sw, q.y, F), sw, e);
-            logU = fma(i2d(e), 0.69314718055994530942, (big ? g : logU) + c);
-            if (--cc == 0) {
-                store(A.ckptB + ck(ci) * LM, w);
-                A.ckptU[ck(ci)] = logU;
-                --ci;
-                cc = C;
-            }
-        };
-        uint32_t p0[KB], e0[KB], h0[KB], p1[KB], e1[KB], h1[KB];
-        float2 q0[KB];
-        double g0[KB], c0[KB];
-        load(0, p0, e0, h0);
-        load(KB, p1, e1, h1);
-        tables(0, p0, h0, nextp, q0, g0, c0);
-        for (uint32_t t0 = 0; t0 + 1 < NAw; t0 += KB) {
-            uint32_t p2[KB], e2[KB], h2[KB];
-            float2 q1[KB];
-            double g1[KB], c1[KB];
-            load(t0 + 2 * KB, p2, e2, h2);
-            tables(t0 + KB, p1, h1, p0[KB - 1], q1, g1, c1);
-            if (__all_sync(0xffffffffu, t0 + KB + 1 <= NA)) {
-#pragma unroll
-                for (uint32_t j = 0; j < KB; ++j) step(e0[j], q0[j], g0[j], c0[j]);
-            } else {
-#pragma unroll
-                for (uint32_t j = 0; j < KB; ++j)
-                    if (t0 + j + 2 <= NA) step(e0[j], q0[j], g0[j], c0[j]);  // a finished chain holds its state
-            }
-#pragma unroll
-            for (uint32_t j = 0; j < KB; ++j) {
-                p0[j] = p1[j]; e0[j] = e1[j]; h0[j] = h1[j]; q0[j] = q1[j]; g0[j] = g1[j]; c0[j] = c1[j];
-                p1[j] = p2[j]; e1[j] = e2[j]; h1[j] = h2[j];
-            }
+                for (uint32_t jj = 0; jj < KB; ++jj) {
+                    const uint32_t j = KB - 1 - jj, k = k0 + j;
+                    Rec rn = r;
+                    double gn = g, cn = c;
+                    if (j > 0) {
+                        rn = read(S, j - 1);
+                        gn = S.g[j - 1][lane];
+                        cn = S.c[j - 1][lane];
+                    }
+                    if (!kStart || k < NAw) {
+                        // the floor's log in units of U: fterm > 0, the floor dominates and the unit
+                        // becomes U rho^n e^fterm; fterm <= -104, it is negligible
+                        const double fterm = g - logU;
+                        const bool big = fterm > 0.0;
+                        const float ex = expf(-fminf(fabsf((float)fterm), 104.f));
+                        const float xs = big ? ex : 1.f;                          // scale of the carried terms
+                        const float F = big ? 1.f : (fterm > -104.0 ? ex : 0.f);  // the floor term
+                        int bits;
+                        update(x, r.m, xs * r.q.x, fmaf(xs * sx, r.q.y, F), sx, bits);
+                        logU = fma(i2d((bits >> 23) - 127), 0.69314718055994530942, (big ? g : logU) + c);
+                        if (kStart && k + 1 >= NA) {  // at or before the chain's last anchor: its start
+                            emission(x, em0);
+                            sx = vsum2<H>(x);
+                            logU = logU0;
+                        }
+                        if (left == 0) {
+                            if (!kStart || k < NA) {
+                                store(ckB, x);
+                                *ckU = logU;
+                            }
+                            left = C;
+                            ckB -= 32 * LM;
+                            ckU -= 32;
+                        }
+                        --left;
+                    }
+                    r = rn;
+                    g = gn;
+                    c = cn;
+                }
+            };
+            if (k0 + KB >= first) steps(std::true_type{});
+            else steps(std::false_type{});
         }
     }
 }
@@ -1220,9 +1298,9 @@ cudaError_t launch_post(const TypedArgs& a, cudaStream_t s) {
 
 template <int LM>
 cudaError_t launch_typed_lm(const TypedArgs& a, bool full, cudaStream_t s) {
-    // a lane per chain, forward and backward warps; one warp per CTA spreads the few warps evenly over the SMs
-    const unsigned long long warps = 2ull * ((a.B + 31) / 32);
-    anchor_chain_kernel<LM><<<(uint32_t)warps, 32, 0, s>>>(a);
+    // a lane per chain; a CTA per direction of a group spreads the few chain warps evenly over the SMs
+    const unsigned long long ctas = 2ull * ((a.B + 31) / 32);
+    anchor_chain_kernel<LM><<<(uint32_t)ctas, kChainThreads, 0, s>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (a.ev_chain_done && (e = cudaEventRecord(a.ev_chain_done, s)) != cudaSuccess) return e;

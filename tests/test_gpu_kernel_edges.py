@@ -1,0 +1,66 @@
+"""Kernels at the sizes where their tiles, blocks and rules of dispatch change
+sides, against the CPU oracle (B200 only).
+
+Bars as in the parity tests: dosage and P(hap=1) within 1e-4 of the FP64
+oracle; argmax alleles equal wherever the oracle's choice is not within 1e-5 of
+the tie threshold.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from swiftimpute_b200 import _native as N
+from swiftimpute_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-4
+
+
+def own_sites(codes_all, counts, seed):
+    """Each target keeps the genotypes of its own random markers, counts[b] of them."""
+    rng = np.random.default_rng(seed)
+    codes = np.full_like(codes_all, 3)
+    for b, n in enumerate(counts):
+        at = rng.choice(codes_all.shape[1], size=n, replace=False)
+        codes[b, at] = codes_all[b, at]
+    return codes
+
+
+def check(engine, panel, pos, codes, L, ne=20000, per_gap=False, **kw):
+    engine.upload_panel(panel)
+    engine.set_map(pos)
+    engine.pbwt_build()
+    p = N.default_params(num_states=L, ne=ne, transition_mode=N.TRANS_PER_GAP if per_gap else N.TRANS_MATRIX0, **kw)
+    got = engine.impute(codes, p, hap_prob=True)
+    pairs = engine.select_states(L)
+    want = oracle.fb_batch(codes, pairs, panel, pos, L, ne, per_gap=per_gap, tie_eps=p.tie_eps)
+    assert np.abs(got["dosage"] - want["dosage"]).max() <= TOL
+    assert np.abs(got["hap_prob"] - want["hap_prob"]).max() <= TOL
+    diff = (got["haps"] != want["haps_argmax"]).any(axis=1)
+    if diff.any():
+        flips = [oracle.fb_batch(codes, pairs, panel, pos, L, ne, per_gap=per_gap, tie_eps=p.tie_eps + d)["haps_argmax"]
+                 for d in (-1e-5, 1e-5)]
+        assert not (diff & ~(flips[0] != flips[1]).any(axis=1)).any()
+    return got
+
+
+# typed markers of the targets of a group: none, one, around the chain's block of
+# eight (and four) anchors, and all; groups whose chains end at different anchors
+@pytest.mark.parametrize("L,spacing", [(3, 1000), (8, 500_000), (8, 1000), (16, 1000), (32, 1000)])
+def test_chain_blocks(engine, L, spacing):
+    M = 300
+    panel, pos, _ = synth.make_panel(M, 512, 20, seed=L, spacing=spacing)
+    counts = [0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 299, 300, 64, 0, 8, 100,
+              40, 41, 42, 43, 44, 300, 1, 2]  # a full group and a partial one
+    codes_all, _, _ = synth.make_targets(panel, len(counts), np.arange(M), seed=L + 1)
+    codes = own_sites(codes_all, counts, seed=L + 2)
+    got = check(engine, panel, pos, codes, L)
+    # a target alone, and all targets of one group equal: the same chain whatever runs beside it
+    p = N.default_params(num_states=L, ne=20000)
+    for b in (0, 8, 22):
+        alone = engine.impute(codes[b:b + 1], p, hap_prob=True)
+        same = engine.impute(np.repeat(codes[b:b + 1], 33, axis=0), p, hap_prob=True)
+        for key in ("dosage", "hap_prob", "haps"):
+            assert np.array_equal(alone[key][0], got[key][b])
+            assert np.array_equal(same[key], np.repeat(got[key][b:b + 1], 33, axis=0))
