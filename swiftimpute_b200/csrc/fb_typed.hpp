@@ -68,8 +68,9 @@ struct TypedArgs {
     // so the lanes of a warp reading the same anchor share cache lines.
     unsigned long long* aoff;        // [G+1] list offsets of the groups (32 x the group's most anchors, or capacities)
     unsigned long long* woff;        // [G+1] window offsets of the groups (likewise)
-    uint32_t* counts;                // [B] anchors of each job (written by the count kernel)
-    uint32_t* segc;                  // [B][nseg] anchors in each segment of kFillSeg markers (count kernel)
+    uint32_t* counts;                // [B] anchors of each job (written by the fill kernel)
+    uint32_t* segc;                  // [nseg][B] anchors in each segment of kFillSeg markers (count kernel)
+    uint32_t split;                  // fill CTAs per segment (set at its launch)
     uint32_t nseg;                   // segments of the longest job: ceil(max_len / kFillSeg)
     uint32_t max_len;                // markers of the longest job (M for a plain batch)
     const uint32_t* cap;             // [B] anchor capacity of each job (a plan), else null: every anchor is listed
@@ -95,7 +96,7 @@ cudaError_t launch_typed_fb(const TypedArgs& a, uint32_t lmax, bool all_full, cu
 size_t typed_post_smem_bytes(uint32_t L, uint32_t T, uint32_t C);
 inline uint32_t typed_groups(uint32_t B) { return (B + 31) / 32; }  // 32-sample groups of the interleaved lists
 constexpr uint32_t kShiftBit = 0x80000000u;                         // apos: no slot matches the call
-constexpr uint32_t kFillSeg = 4096;                                 // markers per warp of the list fill (x 512)
+constexpr uint32_t kFillSeg = 4096;                                 // markers per segment of the lists' counts (x 512)
 inline uint32_t typed_nseg(uint32_t max_len) { return (max_len + kFillSeg - 1) / kFillSeg; }
 // Uneven batches (capi.cu): argument checks, and the region tables and job
 // descriptors of a batch (region sweeps and selections not cached yet run on s).

@@ -105,76 +105,103 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 
 constexpr uint32_t kWarpsPerBlock = 8;
 
-// 16 consecutive codes of a lane (bytes past len read as missing): one 128-bit
-// load when the row is 16-byte aligned and the chunk lies inside it.
-__device__ __forceinline__ uint4 load16(const uint8_t* g, uint32_t base, uint32_t len, bool vec) {
-    if (base >= len) return make_uint4(0x03030303u, 0x03030303u, 0x03030303u, 0x03030303u);
-    if (vec && base + 16 <= len) return *reinterpret_cast<const uint4*>(g + base);
+// Rows of codes are read in 16-byte chunks on absolute 16-byte boundaries, so a
+// row may start anywhere: with a = address % 16, chunk u (a multiple of 16)
+// holds the codes u - a .. u - a + 15 of the row. Codes outside the row read
+// as missing; nothing outside it is read.
+__device__ __forceinline__ uint32_t row_shift(const uint8_t* g) { return (uint32_t)(reinterpret_cast<uintptr_t>(g) & 15u); }
+__device__ __noinline__ uint4 row_edge(const uint8_t* g, uint32_t a, uint32_t u, uint32_t len) {
     uint32_t w[4] = {0x03030303u, 0x03030303u, 0x03030303u, 0x03030303u};
+    if (u < len + a) {  // the row's first or last chunk
 #pragma unroll
-    for (uint32_t j = 0; j < 16; ++j)  // unrolled: the word index is a constant, w stays in registers
-        if (base + j < len)
-            w[j >> 2] = (w[j >> 2] & ~(0xffu << (8 * (j & 3)))) | ((uint32_t)g[base + j] << (8 * (j & 3)));
+        for (uint32_t j = 0; j < 16; ++j)  // unrolled: the word index is a constant, w stays in registers
+            if (u + j >= a && u + j - a < len)
+                w[j >> 2] = (w[j >> 2] & ~(0xffu << (8 * (j & 3)))) | ((uint32_t)__ldg(g + (u + j - a)) << (8 * (j & 3)));
+    }
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
-
-// bit j set when code j of the chunk is below 3 (typed)
-__device__ __forceinline__ uint32_t typed_bits(uint4 c) {
-    const uint32_t ww[4] = {c.x, c.y, c.z, c.w};
-    uint32_t bits = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint32_t lt = __vcmpltu4(ww[q], 0x03030303u);  // 0xff in each byte below 3
-#pragma unroll
-        for (int b = 0; b < 4; ++b) bits |= ((lt >> (8 * b + 7)) & 1u) << (4 * q + b);
-    }
-    return bits;
+__device__ __forceinline__ uint4 row_chunk(const uint8_t* g, uint32_t a, uint32_t u, uint32_t len) {
+    if (u >= a && u - a + 16 <= len) return __ldg(reinterpret_cast<const uint4*>(g + (u - a)));
+    return row_edge(g, a, u, len);
 }
 
-// Per-sample anchor counts: a warp per sample, 16 codes per lane per chunk of
-// 512, the next chunk's load in flight while the current one is counted; the
-// count of every segment of kFillSeg markers goes to segc[s][segment] for the
-// fill, the total (cut to a plan's capacity) to counts[s].
-__global__ void anchor_count_kernel(TypedArgs A) {
-    const uint32_t s = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+// bit 7 of each byte set where the code is below 3 (typed)
+__device__ __forceinline__ uint32_t typed_bytes(uint32_t w) {
+    return ~(((w | 0x80808080u) - 0x03030303u) | w) & 0x80808080u;
+}
+
+// bit j set when code j of the chunk is typed
+__device__ __forceinline__ uint32_t typed_bits(uint4 c) {
+    const uint32_t lo = __dp4a(typed_bytes(c.x) >> 7, 0x08040201u, __dp4a(typed_bytes(c.y) >> 7, 0x80402010u, 0u));
+    const uint32_t hi = __dp4a(typed_bytes(c.z) >> 7, 0x08040201u, __dp4a(typed_bytes(c.w) >> 7, 0x80402010u, 0u));
+    return lo | (hi << 8);
+}
+
+// Anchor counts per segment of kFillSeg markers from a chunk boundary (segment j
+// of a row holds its codes j kFillSeg - a .. (j + 1) kFillSeg - a - 1, the last
+// one the rest): a warp per (sample, segment), its eight 512-byte loads in flight
+// together. Bound by reading the codes: 10,000 x 50,000 in 72 us, 6.9 TB/s of the
+// 6.45 a copy measures (a warp per sample with one load ahead took 163).
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) anchor_count_kernel(TypedArgs A) {
+    const unsigned long long gw = (unsigned long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
+    const uint32_t s = (uint32_t)(gw / A.nseg), seg = (uint32_t)(gw % A.nseg);
     if (s >= A.B) return;
     const View v = view_of(A, s);
-    const bool vec = (reinterpret_cast<uintptr_t>(v.geno) & 15u) == 0;
-    uint32_t* segc = A.segc + (size_t)s * A.nseg;
-    uint32_t n = 0, seg = 0;
-    uint4 cur = load16(v.geno, lane * 16, v.len, vec);
-    for (uint32_t b0 = 0; b0 < v.len; b0 += kFillSeg) {
-        uint32_t c = 0;
-        for (uint32_t base = b0 + lane * 16; base < min(b0 + kFillSeg, v.len); base += 512) {
-            const uint4 nxt = load16(v.geno, base + 512, v.len, vec);
-            uint32_t bits = typed_bits(cur);
-            if (base == 0) bits |= 1u;  // marker 0 is always an anchor
-            c += __popc(bits);
-            cur = nxt;
-        }
+    const uint32_t a = row_shift(v.geno);
+    const uint32_t u0 = seg * kFillSeg;
+    uint32_t n = 0;
+    constexpr uint32_t kIt = kFillSeg / 512;
+    uint4 c[kIt];
+    if (u0 >= a && u0 + kFillSeg - a <= v.len) {  // the whole segment lies inside the row
+        const uint4* p = reinterpret_cast<const uint4*>(v.geno + (u0 - a)) + lane;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if (lane == 0) segc[seg] = c;
-        n += c;
-        ++seg;
+        for (uint32_t i = 0; i < kIt; ++i) c[i] = __ldg(p + 32 * i);
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < kIt; ++i) c[i] = row_chunk(v.geno, a, u0 + 512 * i + 16 * lane, v.len);
     }
-    if (lane == 0) {
-        if (A.cap && n > A.cap[s]) {
-            atomicOr(A.err, 1u);  // the job is cut to its capacity; the host reports it
-            n = A.cap[s];
-        }
-        A.counts[s] = n;
+#pragma unroll
+    for (uint32_t i = 0; i < kIt; ++i)
+        n += __popc(typed_bytes(c[i].x) | (typed_bytes(c[i].y) >> 1) | (typed_bytes(c[i].z) >> 2) | (typed_bytes(c[i].w) >> 3));
+    if (seg + 1 == A.nseg && lane == 0)  // at most 15 codes past the last segment's chunks
+        n += __popc(typed_bits(row_chunk(v.geno, a, u0 + kFillSeg, v.len)));
+    if (seg == 0 && lane == 0 && v.geno[0] >= 3) ++n;  // marker 0 is always an anchor
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) A.segc[(size_t)seg * A.B + s] = n;
+}
+
+// The most anchors of any sample of group g, by one warp (lane = sample).
+__device__ __forceinline__ uint32_t group_most(const uint32_t* __restrict__ segc, uint32_t nseg, uint32_t B, uint32_t g) {
+    const uint32_t s = g * 32 + (threadIdx.x & 31);
+    uint32_t x = 0;
+    if (s < B) {
+#pragma unroll 8
+        for (uint32_t j = 0; j < nseg; ++j) x += __ldg(segc + (size_t)j * B + s);
     }
+    return __reduce_max_sync(0xffffffffu, x);
+}
+
+__global__ void __launch_bounds__(128) anchor_group_kernel(const uint32_t* __restrict__ segc, uint32_t nseg, uint32_t B,
+                                                           unsigned long long* __restrict__ aoff) {
+    const uint32_t g = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (g >= (B + 31) / 32) return;  // whole warp
+    const uint32_t x = group_most(segc, nseg, B, g);
+    if ((threadIdx.x & 31) == 0) aoff[g] = x;
 }
 
 // Exclusive scans over the 32-sample groups of the interleaved lists, in one
 // CTA: a group takes 32 x its most anchors and 32 x its most windows
-// (ceil(count / C)). Entry G holds the totals, also written with the most
-// windows of any sample to host_totals[0..2] (mapped pinned host memory) when
-// given: a copy would queue behind other device-to-host copies on the copy
-// engine.
-__global__ void __launch_bounds__(1024) anchor_scan_kernel(const uint32_t* __restrict__ counts, uint32_t B,
+// (ceil(count / C)). The groups' most anchors are summed up here, or stand in
+// aoff (kGroups false) when anchor_group_kernel ran before: one SM reads the
+// counts of more than kScanGroups groups slower than a second launch costs
+// (313 groups x 13 segments: 43 us in one launch, 6 + 6 in two).
+// Entry G holds the totals, also written with the most windows of any sample to
+// host_totals[0..2] (mapped pinned host memory) when given: a copy would queue
+// behind other device-to-host copies on the copy engine.
+constexpr uint32_t kScanGroups = 64;
+template <bool kGroups>
+__global__ void __launch_bounds__(1024) anchor_scan_kernel(const uint32_t* __restrict__ segc, uint32_t nseg, uint32_t B,
                                                            uint32_t C, unsigned long long* __restrict__ aoff,
                                                            unsigned long long* __restrict__ woff,
                                                            unsigned long long* __restrict__ host_totals) {
@@ -184,11 +211,14 @@ __global__ void __launch_bounds__(1024) anchor_scan_kernel(const uint32_t* __res
     const uint32_t G = (B + 31) / 32;
     const uint32_t per = (G + T - 1) / T;
     const uint32_t g0 = min(G, t * per), g1 = min(G, g0 + per);
-    auto group_max = [&](uint32_t g) {
-        uint32_t x = 0;
-        for (uint32_t b = g * 32; b < min(B, g * 32 + 32); ++b) x = max(x, counts[b]);
-        return x;
-    };
+    if (kGroups) {
+        for (uint32_t g = warp; g < G; g += T >> 5) {
+            const uint32_t x = group_most(segc, nseg, B, g);
+            if (lane == 0) aoff[g] = x;  // until its offset replaces it
+        }
+        __syncthreads();
+    }
+    auto group_max = [&](uint32_t g) { return (uint32_t)aoff[g]; };
     unsigned long long la = 0, lw = 0;
     uint32_t mx = 0;
     for (uint32_t g = g0; g < g1; ++g) {
@@ -222,9 +252,9 @@ __global__ void __launch_bounds__(1024) anchor_scan_kernel(const uint32_t* __res
     __syncthreads();
     unsigned long long ra = sa[warp] + ia - la, rw = sw[warp] + iw - lw;
     for (uint32_t g = g0; g < g1; ++g) {
+        const uint32_t x = group_max(g);
         aoff[g] = ra;
         woff[g] = rw;
-        const uint32_t x = group_max(g);
         ra += 32ull * x;
         rw += 32ull * ((x + C - 1) / C);
     }
@@ -242,101 +272,143 @@ __global__ void __launch_bounds__(1024) anchor_scan_kernel(const uint32_t* __res
 
 // Anchor lists: marker position (with the "no slot matches" flag, which
 // scales every slot by e^-999, counted in beta's unit, in bit 31) and emission
-// mask over the slots, in marker order; marker 0 is always an anchor. A warp
-// (one CTA) fills one segment of kFillSeg markers of the 32 samples of a
-// group, lane = sample: chunks of 32 rows x 256 codes (and, for a plain batch,
-// the chunk's slot masks) come into shared memory by cp.async, the next chunk
-// in flight while each lane scans its own row of the current one, and lanes
-// that meet their anchors in step (shared typed positions) write whole
-// 128-byte lines of the interleaved lists. A lane's first entry of the segment
-// is the sum of its earlier segments' counts.
-constexpr uint32_t kFillChunk = 256;                 // markers per staged chunk
-constexpr uint32_t kFillRow = kFillChunk + 16;        // row stride in shared memory (bytes): conflict-free 128-bit reads
-constexpr size_t kFillBuf = 32 * kFillRow + kFillChunk * sizeof(SlotMasks);  // codes of 32 rows, the chunk's slot masks
-constexpr size_t kFillSmem = 2 * kFillBuf + 32 * 16;  // two chunk buffers and the row descriptors
+// mask over the slots, in marker order; marker 0 is always an anchor. A CTA
+// fills one segment of the 32 samples of a group, 512 markers of every row at a
+// time: a warp takes four rows, each lane 16 codes of one, and puts the typed
+// ones (a warp scan gives their places) into the row's list in shared memory;
+// then the warps write entry after entry of all 32 rows, lane = row, so lanes
+// at the same entry (samples of one array) write whole 128-byte lines of the
+// interleaved lists. The next 512 codes of the rows are on their way meanwhile.
+// A row's first entry of the segment is the sum of its earlier segments' counts.
+// A batch of few groups is split further, A.split CTAs a segment: each counts the
+// part of the segment before its own again.
+// Bound by instruction issue (finding and placing the typed codes, about 110
+// warp instructions per 512): 10,000 x 50,000 codes with 2,942 typed in 231 us, of
+// which reading them once would be 78. A warp per group that walked its rows lane
+// by lane took 300 us, and four to ten times as long where rows start off 16-byte
+// boundaries (single-byte loads): the lists of 2,003 x 30,011 took 403 us in all
+// and take 93, those of 1,500 x 6,007 302 and 56, those of one target 87 and 40
+// (most of it the host's wait for the totals).
+constexpr uint32_t kFillChunk = 512;
+constexpr uint32_t kFillWarps = 8;
+constexpr uint32_t kFillStride = kFillChunk + 2;  // list stride (entries): an odd number of words, no bank conflicts
 
-__global__ void __launch_bounds__(32) anchor_fill_kernel(TypedArgs A) {
-    extern __shared__ __align__(16) unsigned char fsm[];
-    const uint32_t lane = threadIdx.x;
+__global__ void __launch_bounds__(32 * kFillWarps, 4) anchor_fill_kernel(TypedArgs A) {
+    __shared__ uint16_t list[32][kFillStride];  // position in the chunk | code << 9
+    __shared__ uint32_t cnt[32], part[kFillWarps][32];
+    __shared__ uint4 rowd[32];  // {ptr lo, ptr hi, len, -}
+    constexpr uint32_t kRows = 32 / kFillWarps;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t G = (A.B + 31) / 32;
-    const uint32_t g = blockIdx.x % G, seg = blockIdx.x / G;
-    const uint32_t s = g * 32 + lane;
-    uint4* rowd = reinterpret_cast<uint4*>(fsm + 2 * kFillBuf);  // [32] {ptr lo, ptr hi, len, 16-byte aligned}
+    const uint32_t g = blockIdx.x % G, seg = blockIdx.x / G / A.split, sub = blockIdx.x / G % A.split;
+    const uint32_t s = g * 32 + lane;  // lane = row
     View v{};
-    uint32_t len = 0, at = 0, lim = 0;
+    uint32_t lim = 0;
     if (s < A.B) {
         v = view_of(A, s);
-        len = v.len;
-        const uint32_t* segc = A.segc + (size_t)s * A.nseg;
-        for (uint32_t j = 0; j < seg; ++j) at += segc[j];
-        lim = A.counts[s];  // a plan's capacity cut, else every anchor
+        lim = A.cap ? A.cap[s] : 0xffffffffu;
+        uint32_t sum = 0;
+        for (uint32_t j = warp; j < seg; j += kFillWarps) sum += A.segc[(size_t)j * A.B + s];
+        part[warp][lane] = sum;
     }
-    const uint32_t m0 = seg * kFillSeg;
-    const uint32_t mlast = __reduce_max_sync(0xffffffffu, len);
-    if (m0 >= mlast) return;  // whole warp: no row reaches this segment
-    const unsigned long long gp = reinterpret_cast<unsigned long long>(v.geno);
-    rowd[lane] = make_uint4((uint32_t)gp, (uint32_t)(gp >> 32), len, (gp & 15u) == 0 ? 1u : 0u);
-    __syncwarp();
+    const uint32_t a = row_shift(v.geno);
+    if (warp == 0) {
+        const unsigned long long gp = reinterpret_cast<unsigned long long>(v.geno);
+        rowd[lane] = make_uint4((uint32_t)gp, (uint32_t)(gp >> 32), s < A.B ? v.len : 0u, 0u);
+    }
+    __syncthreads();
+    uint32_t at = 0;
+    if (s < A.B) {
+#pragma unroll
+        for (uint32_t w = 0; w < kFillWarps; ++w) at += part[w][lane];
+        if (warp == 0 && seg + 1 == A.nseg && sub == 0) {
+            const uint32_t n = at + A.segc[(size_t)seg * A.B + s];
+            if (n > lim) atomicOr(A.err, 1u);  // the job is cut to its capacity; the host reports it
+            A.counts[s] = min(n, lim);
+        }
+    }
+    const uint32_t ulast = __reduce_max_sync(0xffffffffu, s < A.B ? v.len + a : 0u);
+    const uint32_t us = seg * kFillSeg, u0 = us + sub * (kFillSeg / A.split);
+    const bool tail = seg + 1 == A.nseg && sub + 1 == A.split;
+    const uint32_t u1 = tail ? ulast : min(u0 + kFillSeg / A.split, ulast);
+    if (u0 >= u1) return;  // whole CTA: no row reaches this part
     const uint32_t lmask = lmask_of(v.r.L);
     const unsigned long long lb = A.aoff[g] + lane;
-    // a plain batch shares one slot-mask table: its chunk is staged beside the codes
-    const bool stage_masks = A.samples == nullptr;
-    const SlotMasks* gmasks = A.reg0.masks;
-    // chunk at c0 into buffer b: rows 2 it + lane / 16, bytes 16 (lane % 16) .. + 16, and the masks
-    auto issue = [&](uint32_t c0, unsigned char* b) {
-        const uint32_t mm = c0 + 16 * (lane & 15);
-#pragma unroll 4
-        for (uint32_t it = 0; it < 16; ++it) {
-            const uint32_t r = 2 * it + (lane >> 4);
-            const uint4 d = rowd[r];
-            const uint8_t* gr = reinterpret_cast<const uint8_t*>(((unsigned long long)d.y << 32) | d.x);
-            unsigned char* dst = b + r * kFillRow + 16 * (lane & 15);
-            if (d.w && mm + 16 <= d.z) cp_async16(dst, gr + mm);
-            else *reinterpret_cast<uint4*>(dst) = load16(gr, mm, d.z, d.w != 0);  // a ragged or unaligned row
-        }
-        if (stage_masks) {
-            SlotMasks* sm = reinterpret_cast<SlotMasks*>(b + 32 * kFillRow);
-            for (uint32_t i = lane; i < kFillChunk && c0 + i < A.M; i += 32) cp_async16(sm + i, gmasks + c0 + i);
-        }
-        cp_async_commit();
+    const uint8_t* rp[kRows];
+    uint32_t rl[kRows];
+#pragma unroll
+    for (uint32_t i = 0; i < kRows; ++i) {
+        const uint4 d = rowd[warp * kRows + i];
+        rp[i] = reinterpret_cast<const uint8_t*>(((unsigned long long)d.y << 32) | d.x);
+        rl[i] = d.z;
+    }
+    uint4 cur[kRows];
+    auto load = [&](uint32_t c0) {
+#pragma unroll
+        for (uint32_t i = 0; i < kRows; ++i) cur[i] = row_chunk(rp[i], row_shift(rp[i]), c0 + 16 * lane, rl[i]);
     };
-    const uint32_t cend = min(m0 + kFillSeg, mlast);
-    issue(m0, fsm);
-    uint32_t bi = 0;
-    for (uint32_t c0 = m0; c0 < cend; c0 += kFillChunk, bi ^= 1) {
-        if (c0 + kFillChunk < cend) {
-            issue(c0 + kFillChunk, fsm + (bi ^ 1) * kFillBuf);
-            cp_async_wait_group<1>();  // this lane's copies of the current chunk have landed
-        } else {
-            cp_async_wait_group<0>();
+    load(u0);
+    if (sub) {  // the segment's markers before u0
+#pragma unroll
+        for (uint32_t i = 0; i < kRows; ++i) {
+            uint32_t n = 0;
+#pragma unroll 4
+            for (uint32_t u = us + 16 * lane; u < u0; u += kFillChunk)
+                n += __popc(typed_bits(row_chunk(rp[i], row_shift(rp[i]), u, rl[i])));
+            if (us + lane == 0 && rl[i] && rp[i][0] >= 3) ++n;
+            n = __reduce_add_sync(0xffffffffu, n);
+            if (lane == 0) cnt[warp * kRows + i] = n;
         }
-        __syncwarp();  // ... and every lane's
-        if (c0 < len) {
-            const unsigned char* buf = fsm + bi * kFillBuf;
-            const unsigned char* row = buf + lane * kFillRow;
-            const SlotMasks* sm = reinterpret_cast<const SlotMasks*>(buf + 32 * kFillRow);
-            for (uint32_t q = 0; q < kFillChunk / 16; ++q) {
-                const uint4 x = *reinterpret_cast<const uint4*>(row + 16 * q);
-                uint32_t bits = typed_bits(x);
-                const uint32_t base = c0 + 16 * q;
-                if (base == 0) bits |= 1u;
-                while (bits) {
-                    const uint32_t j = __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    const uint32_t m = base + j;
-                    if (at < lim) {
-                        uint32_t sh;
-                        const uint32_t w = j < 8 ? (j < 4 ? x.x : x.y) : (j < 12 ? x.z : x.w);
-                        const SlotMasks mk = stage_masks ? sm[m - c0] : v.r.masks[m];
-                        const uint32_t em = emission_mask((w >> (8 * (j & 3))) & 0xffu, mk, lmask, &sh);
-                        A.apos[lb + 32ull * at] = m | (sh ? kShiftBit : 0u);
-                        A.aem[lb + 32ull * at] = em;
-                    }
-                    ++at;
-                }
+        __syncthreads();
+        at += cnt[lane];
+        __syncthreads();
+    }
+    for (uint32_t c0 = u0; c0 < u1; c0 += kFillChunk) {
+        uint32_t bits[kRows], incl[kRows / 2];  // counts of two rows share a word (a chunk has at most 512)
+#pragma unroll
+        for (uint32_t i = 0; i < kRows; ++i) {
+            bits[i] = typed_bits(cur[i]);
+            if (c0 + lane == 0 && rl[i]) bits[i] |= 1u << row_shift(rp[i]);  // marker 0
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kRows / 2; ++i) incl[i] = __popc(bits[2 * i]) | __popc(bits[2 * i + 1]) << 16;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+            for (uint32_t i = 0; i < kRows / 2; ++i) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl[i], o);
+                if (lane >= (uint32_t)o) incl[i] += y;
             }
         }
-        __syncwarp();  // the buffer is read before it is refilled
+#pragma unroll
+        for (uint32_t i = 0; i < kRows; ++i) {
+            const uint4 x = cur[i];
+            const uint32_t end = i & 1 ? incl[i / 2] >> 16 : incl[i / 2] & 0xffffu;
+            if (lane == 31) cnt[warp * kRows + i] = end;
+            uint16_t* to = &list[warp * kRows + i][end - __popc(bits[i])];
+            for (uint32_t b = bits[i]; b; b &= b - 1) {
+                const uint32_t j = __ffs(b) - 1;
+                const uint32_t w = j < 8 ? (j < 4 ? x.x : x.y) : (j < 12 ? x.z : x.w);
+                const uint32_t code = min((w >> (8 * (j & 3))) & 0xffu, 3u);
+                *to++ = (uint16_t)(16 * lane + j | code << 9);
+            }
+        }
+        if (c0 + kFillChunk < u1) load(c0 + kFillChunk);
+        __syncthreads();
+        const uint32_t n = cnt[lane], most = __reduce_max_sync(0xffffffffu, n);
+#pragma unroll 2
+        for (uint32_t k = warp; k < most; k += kFillWarps) {
+            if (k < n && at + k < lim) {
+                const uint32_t e = list[lane][k];
+                const uint32_t m = c0 + (e & 511u) - a;
+                uint32_t sh;
+                const uint32_t em = emission_mask(e >> 9, v.r.masks[m], lmask, &sh);
+                A.apos[lb + 32ull * (at + k)] = m | (sh ? kShiftBit : 0u);
+                A.aem[lb + 32ull * (at + k)] = em;
+            }
+        }
+        at += n;
+        __syncthreads();  // the lists are read before they are refilled
     }
 }
 
@@ -1319,24 +1391,37 @@ size_t typed_post_smem_bytes(uint32_t L, uint32_t T, uint32_t C) {
     return (size_t)(T / 32) * post_warp_bytes(fb_lmax(L), C, true);
 }
 
-cudaError_t launch_anchor_lists_count(const TypedArgs& a, cudaStream_t s) {
-    anchor_count_kernel<<<(a.B + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, s>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    anchor_scan_kernel<<<1, 1024, 0, s>>>(a.counts, a.B, a.C, a.aoff, a.woff, a.host_totals);
+cudaError_t launch_anchor_count_only(const TypedArgs& a, cudaStream_t s) {
+    const unsigned long long warps = (unsigned long long)a.B * a.nseg;
+    const unsigned long long grid = (warps + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+    anchor_count_kernel<<<(uint32_t)grid, kWarpsPerBlock * 32, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_anchor_count_only(const TypedArgs& a, cudaStream_t s) {
-    anchor_count_kernel<<<(a.B + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, s>>>(a);
+cudaError_t launch_anchor_lists_count(const TypedArgs& a, cudaStream_t s) {
+    const cudaError_t e = launch_anchor_count_only(a, s);
+    if (e != cudaSuccess) return e;
+    const uint32_t G = typed_groups(a.B);
+    if (G <= kScanGroups) {
+        anchor_scan_kernel<true><<<1, 1024, 0, s>>>(a.segc, a.nseg, a.B, a.C, a.aoff, a.woff, a.host_totals);
+    } else {
+        anchor_group_kernel<<<(G + 3) / 4, 128, 0, s>>>(a.segc, a.nseg, a.B, a.aoff);
+        anchor_scan_kernel<false><<<1, 1024, 0, s>>>(a.segc, a.nseg, a.B, a.C, a.aoff, a.woff, a.host_totals);
+    }
     return cudaGetLastError();
 }
 
 cudaError_t launch_anchor_lists_fill(const TypedArgs& a, cudaStream_t s) {
-    const unsigned long long grid = (unsigned long long)typed_groups(a.B) * a.nseg;  // a warp per CTA
+    // split the segments while they would leave SMs without four CTAs (a small batch is a few chunks of latency)
+    const unsigned long long parts = (unsigned long long)typed_groups(a.B) * a.nseg;
+    TypedArgs f = a;
+    f.split = 1;
+    while (f.split < kFillSeg / kFillChunk && parts * f.split < 4 * 148) f.split *= 2;
+    const unsigned long long grid = parts * f.split;
     if (grid == 0) return cudaSuccess;
     if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-    anchor_fill_kernel<<<(uint32_t)grid, 32, kFillSmem, s>>>(a);
+    anchor_fill_kernel<<<(uint32_t)grid, 32 * kFillWarps, 0, s>>>(f);
     return cudaGetLastError();
 }
 

@@ -64,3 +64,19 @@ def test_chain_blocks(engine, L, spacing):
         for key in ("dosage", "hap_prob", "haps"):
             assert np.array_equal(alone[key][0], got[key][b])
             assert np.array_equal(same[key], np.repeat(got[key][b:b + 1], 33, axis=0))
+
+
+# rows that start anywhere, lengths around the lists' chunks (16, 512) and segments (4,096), batches
+# around a group, typed and untyped first and last markers, rows without any typed marker
+@pytest.mark.parametrize("M", [1, 2, 15, 16, 17, 31, 33, 497, 511, 513, 1023, 4095, 4096, 4097, 4111, 4112, 8191, 8209])
+def test_list_rows(engine, M):
+    B = 33 if M < 1000 else 5
+    panel, pos, _ = synth.make_panel(M, 256, 20, seed=M, spacing=500_000)
+    codes_all, _, _ = synth.make_targets(panel, B, np.arange(M), seed=M + 1, het_range=(0.0, 1.0))
+    rng = np.random.default_rng(M + 2)
+    codes = own_sites(codes_all, rng.integers(0, min(M, 600) + 1, B), seed=M + 3)
+    codes[0] = 3
+    codes[1] = codes_all[1]
+    codes[2, -1] = codes_all[2, -1]
+    codes[3] = np.where(codes[3] == 3, rng.integers(3, 256, M), codes[3])  # any byte above 2 is a missing call
+    check(engine, panel, pos, codes, 8)
