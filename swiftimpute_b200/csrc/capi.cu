@@ -258,8 +258,6 @@ void default_tiles(uint32_t L, uint32_t* T, uint32_t* C) {
     *T = lm <= 8 ? 64 : 32;
 }
 
-constexpr uint32_t kTabN = 4096;
-
 // Closed-form run coefficients for (c, delta, L) in FP64 (fb_typed.hpp),
 // cached per (transition, L).
 si_status tables_for(si_ctx* ctx, const LinTrans& t0, uint32_t L, TypedTables* out) {
@@ -275,8 +273,8 @@ si_status tables_for(si_ctx* ctx, const LinTrans& t0, uint32_t L, TypedTables* o
         const double lr = std::log(rho);
         const int regime = std::fabs(rho - 1.0) < 1e-15 ? 2 : (rho < 1.0 ? 0 : 1);
         const double lgc = regime == 0 ? std::log1p(-rho) : (regime == 1 ? std::log(rho - 1.0) : 0.0);
-        // QS [n] {Q, S}; then the pair tables {Q_n, Q_n+1, S_n, S_n+1} and
-        // {Q_n, Q_n-1, S_n, S_n-1} (index 0: Q_0, S_0 twice) for two consecutive cells
+        // QS [n] {Q, S}; then for two consecutive cells up [n] {Q_n, Q_n+1, S_n, S_n+1}
+        // and dg [n] {Q_n, Q_n-1, S_n, S_n-1} (index 0: Q_0, S_0 twice) with G beside it
         std::vector<float> QS(2 * kTabN + 12 * kTabN);
         std::vector<double> G(kTabN);
         std::vector<float> qf(kTabN + 1), sf(kTabN + 1);
@@ -287,26 +285,25 @@ si_status tables_for(si_ctx* ctx, const LinTrans& t0, uint32_t L, TypedTables* o
             sf[n] = (float)(om / (double)L);
         }
         float* up = QS.data() + 2 * kTabN;
-        float* dn = up + 4 * kTabN;
+        float* dg = up + 4 * kTabN;
         for (uint32_t n = 0; n < kTabN; ++n) {
             QS[2 * n] = qf[n];
             QS[2 * n + 1] = sf[n];
             up[4 * n] = qf[n]; up[4 * n + 1] = qf[n + 1]; up[4 * n + 2] = sf[n]; up[4 * n + 3] = sf[n + 1];
             const uint32_t b = n ? n - 1 : 0;
-            dn[4 * n] = qf[n]; dn[4 * n + 1] = qf[b]; dn[4 * n + 2] = sf[n]; dn[4 * n + 3] = sf[b];
+            dg[8 * n] = qf[n]; dg[8 * n + 1] = qf[b]; dg[8 * n + 2] = sf[n]; dg[8 * n + 3] = sf[b];
             if (n == 0) G[n] = -INFINITY;
             else if (regime == 0) G[n] = -(double)n * lr + std::log(-std::expm1((double)n * lr)) - lgc;
             else if (regime == 1) G[n] = std::log(-std::expm1(-(double)n * lr)) - lgc;
             else G[n] = std::log((double)n);
         }
-        // Gdn [n] {hi G_n, hi G_n-1, lo G_n, lo G_n-1}: G as a float pair, so the floor's
+        // {hi G_n, hi G_n-1, lo G_n, lo G_n-1}: G as a float pair, so the floor's
         // log farg' + G_j (nearly cancelling where the floor matters) is formed in FP32
-        float* gd = dn + 4 * kTabN;
         auto hi = [&](uint32_t n) { return n == 0 ? -1e30f : (float)G[n]; };
         auto lo = [&](uint32_t n) { return n == 0 ? 0.f : (float)(G[n] - (double)(float)G[n]); };
         for (uint32_t n = 0; n < kTabN; ++n) {
             const uint32_t b = n ? n - 1 : 0;
-            gd[4 * n] = hi(n); gd[4 * n + 1] = hi(b); gd[4 * n + 2] = lo(n); gd[4 * n + 3] = lo(b);
+            dg[8 * n + 4] = hi(n); dg[8 * n + 5] = hi(b); dg[8 * n + 6] = lo(n); dg[8 * n + 7] = lo(b);
         }
         si_status st = dev_alloc(ctx, ts.QS, QS.size() * 4);
         if (st == SI_OK) st = dev_alloc(ctx, ts.G, kTabN * 8);
@@ -323,9 +320,8 @@ si_status tables_for(si_ctx* ctx, const LinTrans& t0, uint32_t L, TypedTables* o
         ts.consts[3] = regime;
     }
     out->QS = (const float2*)ts.QS.ptr; out->G = (const double*)ts.G.ptr;
-    out->QSup = (const float4*)((const float*)ts.QS.ptr + 2 * kTabN);
-    out->QSdn = out->QSup + kTabN;
-    out->Gdn = out->QSdn + kTabN;
+    out->up = (const float4*)((const float*)ts.QS.ptr + 2 * kTabN);
+    out->dg = out->up + kTabN;
     out->NT = kTabN; out->log2q = (float)ts.consts[0]; out->invL = 1.0f / (float)L;
     out->lr = ts.consts[1]; out->lgc = ts.consts[2]; out->regime = (int)ts.consts[3];
     return SI_OK;

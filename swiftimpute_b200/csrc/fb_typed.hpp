@@ -8,14 +8,15 @@ namespace si {
 // Closed-form coefficients for runs of untyped markers under one transition
 // (c, delta), computed in FP64 on the host: q = delta / rho, rho = delta + L c,
 // QS[n] = {Q[n], S[n]} = {q^n, (1 - q^n) / L}, G[n] = log sum_{k=1..n} rho^-k;
-// for two consecutive cells QSup[n] = {Q[n], Q[n+1], S[n], S[n+1]} and
-// QSdn[n] = {Q[n], Q[n-1], S[n], S[n-1]}; Gdn[n] = {hi G[n], hi G[n-1],
-// lo G[n], lo G[n-1]}, G as a float pair hi + lo (G[0] = -inf stands as -1e30).
+// for two consecutive cells up[n] = {Q[n], Q[n+1], S[n], S[n+1]} and the pair
+// dg[2n] = {Q[n], Q[n-1], S[n], S[n-1]}, dg[2n+1] = {hi G[n], hi G[n-1], lo G[n],
+// lo G[n-1]}, G as a float pair hi + lo (G[0] = -inf stands as -1e30); kTabN
+// entries of each.
+constexpr uint32_t kTabN = 4096;
 struct TypedTables {
     const float2* QS;
-    const float4* QSup;
-    const float4* QSdn;
-    const float4* Gdn;
+    const float4* up;
+    const float4* dg;
     const double* G;
     uint32_t NT;
     float log2q;
@@ -55,6 +56,7 @@ struct TypedArgs {
     uint32_t M;                      // markers per sample of a plain batch
     uint32_t C, threads;             // anchors per window (backward checkpoints), posterior CTA size
     uint32_t K;                      // windows per posterior group (forward checkpoints every K windows)
+    uint32_t stage;                  // posterior CTAs hold slot data in shared memory (set at its launch)
     uint32_t max_windows;            // most windows of any sample (posterior grid)
     int sampling;
     float tie_eps;

@@ -451,49 +451,34 @@ __device__ __forceinline__ double chain_end_logU(const Tabs& tb, uint32_t n) {
     return (double)n * tb.lr + (f > 30.0 ? f + log1p(exp(-f)) : log1p(exp(f)));
 }
 
+// One backward step of a window's rebuild over a run of n markers to the anchor
+// with emission em (sh: no slot matches its call). The floor's log in units of
+// U: fterm > 0, the floor dominates and the unit becomes U rho^n e^fterm;
+// fterm <= -104, it is negligible. No branch: a warp's lanes differ in this.
 template <int LM>
 __device__ __forceinline__ void backward_step(const Tabs& tb, uint32_t n, float (&w)[LM], double& logU, uint32_t em,
-                                              uint32_t sh, uint32_t lmask) {
+                                              uint32_t sh) {
     const float2 qs = tabQS(tb, n);
-    const float Qn = qs.x, Sn = qs.y;
     const float sw = vsum<LM>(w);
     const double fterm = -999.0 - logU + tabG(tb, n);
-    if (fterm > 0.0) {
-        // the floor dominates: unit becomes U rho^n e^fterm
-        const float g = expf(-(float)fmin(fterm, 100.0));
-        const float base = fmaf(g * sw, Sn, 1.0f);
-        const float gq = g * Qn;
+    const bool big = fterm > 0.0;
+    const float ft = (float)fterm;
+    const float ex = expf(big ? -fminf(ft, 100.f) : ft);
+    const float xs = big ? ex : 1.f;                          // scale of the carried terms
+    const float F = big ? 1.f : (fterm > -104.0 ? ex : 0.f);  // the floor term
+    const float base = fmaf(xs * sw, qs.y, F);
+    const float g = xs * qs.x;
 #pragma unroll
-        for (int k = 0; k < LM; ++k) w[k] = ((em >> k) & 1u) ? fmaf(gq, w[k], base) : 0.f;
-        logU += (double)n * tb.lr + fterm;
-    } else {
-        const float F = fterm > -104.0 ? expf((float)fterm) : 0.f;
-        const float base = fmaf(sw, Sn, F);
-#pragma unroll
-        for (int k = 0; k < LM; ++k) w[k] = ((em >> k) & 1u) ? fmaf(Qn, w[k], base) : 0.f;
-        logU += (double)n * tb.lr;
-    }
-    (void)lmask;
-    logU -= 999.0 * (double)sh;
+    for (int k = 0; k < LM; ++k) w[k] = ((em >> k) & 1u) ? fmaf(g, w[k], base) : 0.f;
+    const double dn = u2d(n);
+    logU = big ? logU + fma(dn, tb.lr, fterm) : fma(dn, tb.lr, logU);
+    logU -= sh ? 999.0 : 0.0;
     const float s = vsum<LM>(w);
     const int e = exp2_of(s);
     const float sc = pow2_neg(e);
 #pragma unroll
     for (int k = 0; k < LM; ++k) w[k] *= sc;
-    logU += (double)e * 0.69314718055994530942;
-}
-
-template <int LM>
-__device__ __forceinline__ void forward_step(const Tabs& tb, uint32_t n, float (&a)[LM], uint32_t em) {
-    const float2 qs = tabQS(tb, n);
-    const float Qn = qs.x, Sn = qs.y;
-    const float base = vsum<LM>(a) * Sn;
-#pragma unroll
-    for (int k = 0; k < LM; ++k) a[k] = ((em >> k) & 1u) ? fmaf(Qn, a[k], base) : 0.f;
-    const int e = exp2_of(vsum<LM>(a));
-    const float sc = pow2_neg(e);
-#pragma unroll
-    for (int k = 0; k < LM; ++k) a[k] *= sc;
+    logU = fma(i2d(e), 0.69314718055994530942, logU);
 }
 
 template <int LM>
@@ -829,12 +814,23 @@ __global__ void __launch_bounds__(kChainThreads, LM <= 16 ? 5 : 3) anchor_chain_
 // per-lane staging area with cp.async while the previous window is walked.
 // With a' and w' of unit sum, a cell i markers after pos[k] and j = pos[k+1]
 // - m before the next anchor has alpha_l ~ Q[i] a'_l + S[i] and beta_l ~
-// Q[j] w'_l + S[j] (+ floor). Lanes whose samples share typed positions (an
-// array's sites, every batch of the benchmark workloads) step through the
-// same markers, so the per-marker slot data are warp-uniform loads; other
-// lanes still work, with divergent anchor steps. Outputs are staged in a
-// per-warp tile [32 samples][32 markers] in shared memory and leave as row
-// segments of 32 consecutive markers.
+// Q[j] w'_l + S[j] (+ floor). Outputs are staged in a per-warp tile [32
+// samples][32 markers] in shared memory and leave as row segments of 32
+// consecutive markers.
+//
+// Two walks. If every sample of the CTA has the same anchors in the group (an
+// array's sites; the kernel looks, one load an anchor), all its lanes step
+// through the same markers: control and addresses are the warp's, the CTA stages
+// the markers' slot data and the head of the run tables in shared memory, a tile
+// ahead, and the floor is one branch-free form for all lanes. Otherwise every
+// lane walks by itself. The arithmetic of a cell is the same, bit for bit.
+// Bound: instruction issue. A pair of cells takes about 140 warp instructions at
+// L = 8 (24 f32x2 operations for the slots, 15 for the sums, 47 for the argmax,
+// 20 for the floor), an anchor about 300. Launch times, one walk for all before
+// -> now: 10,000 x 50,000 (L = 8) 4.06 -> 2.35 ms (writing its 3 GB would take
+// 0.47); 2,003 x 30,011 0.76 -> 0.41; 4,000 x 20,000 (L = 16) 1.27 -> 0.68; 1,500
+// x 6,007 (L = 32, alleles only) 0.22 -> 0.18; one target x 1,644 98 -> 57 us;
+// 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 1.12 ms.
 
 // high word of farg' for a uniform run and for a negligible floor
 constexpr uint32_t kInfHi = 0x7ff00000u;
@@ -843,6 +839,12 @@ constexpr uint32_t kNegInfHi = 0xfff00000u;
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -878,21 +880,33 @@ __device__ __forceinline__ void pick_pair(const float2 (&p2)[LM], float keep, ui
         bx = __funnelshift_l(__float_as_uint(d.x), bx, 1);
         by = __funnelshift_l(__float_as_uint(d.y), by, 1);
     }
-    constexpr uint32_t kLow = LM >= 32 ? 0xffffffffu : ((1u << LM) - 1u);
-    k0 = (uint32_t)__clz(~bx & kLow) - (32u - LM);
-    k1 = (uint32_t)__clz(~by & kLow) - (32u - LM);
+    constexpr uint32_t kTop = LM >= 32 ? 1u : 1u << (32 - LM);  // slot l's bit at 31 - l, the bits below clear
+    k0 = (uint32_t)__clz(~bx * kTop);
+    k1 = (uint32_t)__clz(~by * kTop);
 }
 
+// x >> k, 0 for k = 32 (no slot picked)
+__device__ __forceinline__ uint32_t shr(uint32_t x, uint32_t k) { return __funnelshift_rc(x, 0u, k); }
+
 // Shared memory of one warp: backward records [C][LM/4][32] float4 and
-// [C][32] {farg' lo, farg' hi, run end, end emission}; the flush descriptors
-// [2][32] uint4; the dosage tile [32][36] f32, the allele tile [64][36] u8
+// [C][32] {farg' lo, farg' hi, run end, end emission}; the dosage tile [32][36] f32, the allele tile [64][36] u8
 // (rows 2r and 2r + 1: the two haplotypes of lane r) and, for P(hap=1),
 // [32][34] f32x2; the staging area of the next window: end checkpoint
 // [LM/4][32] float4 and [32] f64, list entries [C+1][32] positions and
 // [C+1][32] emission masks.
 __host__ __device__ constexpr size_t post_warp_bytes(uint32_t LM, uint32_t C, bool hprob) {
-    return (size_t)C * LM * 128 + (size_t)C * 512 + 1024 + 32 * 36 * 4 + 64 * 36 + (hprob ? 32 * 34 * 8 : 0) +
+    return (size_t)C * LM * 128 + (size_t)C * 512 + 32 * 36 * 4 + 64 * 36 + (hprob ? 32 * 34 * 8 : 0) +
            (size_t)LM * 128 + 256 + 2 * ((size_t)C + 1) * 128;
+}
+
+// In front of the warps' parts, when A.stage: the head of the run tables (up and
+// dg, kPostTab entries), two tiles of slot data (32 markers' masks and, where
+// dosage is written, weights), and what warp 0 walks.
+constexpr uint32_t kPostTab = 64;
+// 32 slots' weights would take a CTA an SM: they are read where they lie
+__host__ __device__ constexpr bool post_stage_weights(uint32_t LM, bool dos) { return dos && LM <= 16; }
+__host__ __device__ constexpr size_t post_cta_bytes(uint32_t LM, bool dos) {
+    return kPostTab * 48 + 2 * (32 * sizeof(SlotMasks) + (post_stage_weights(LM, dos) ? 32 * (size_t)LM * 8 : 0)) + 32;
 }
 
 struct Staging {
@@ -908,10 +922,21 @@ __device__ __forceinline__ void stage_window(const TypedArgs& A, const uint32_t*
                                              unsigned long long wb, uint32_t NA, uint32_t w, const Staging& st,
                                              uint32_t lane) {
     const uint32_t C = A.C, k0 = w * C, k1 = min(k0 + C, NA);
-    const uint32_t kl = min(k1, NA - 1);
-    for (uint32_t k = k0; k <= kl; ++k) {
-        cp_async4(st.P + (k - k0) * 32 + lane, apos + 32ull * k);
-        cp_async4(st.E + (k - k0) * 32 + lane, aem + 32ull * k);
+    const uint32_t* p = apos + 32ull * k0;
+    const uint32_t* e0 = aem + 32ull * k0;
+    uint32_t* sp = st.P + lane;
+    uint32_t* se = st.E + lane;
+    if (C == 2 && k1 < NA) {
+#pragma unroll
+        for (uint32_t n = 0; n < 3; ++n) {
+            cp_async4(sp + 32 * n, p + 32 * n);
+            cp_async4(se + 32 * n, e0 + 32 * n);
+        }
+    } else {
+        for (uint32_t n = min(k1, NA - 1) - k0 + 1; n; --n, p += 32, e0 += 32, sp += 32, se += 32) {
+            cp_async4(sp, p);
+            cp_async4(se, e0);
+        }
     }
     if (k1 < NA) {
         const unsigned long long e = wb + 32ull * (w + 1);
@@ -921,6 +946,24 @@ __device__ __forceinline__ void stage_window(const TypedArgs& A, const uint32_t*
         cp_async8(st.U + lane, A.ckptU + e);
     }
     cp_async_commit();
+}
+
+// The backward record of a run of n markers from the vector bv of its end
+// anchor (at position pk, emission em) and the log of that vector's unit.
+template <int LM>
+__device__ __forceinline__ void write_record(const Tabs& tb, uint32_t n, const float (&bv)[LM], double logU, uint32_t pk,
+                                             uint32_t em, float4* recW, uint4* recF) {
+    const float sw = vsum<LM>(bv);
+    const double farg = -999.0 - logU;
+    const double f = farg - (double)logf(sw);
+    uint32_t lo = (uint32_t)__double2loint(f), hi = (uint32_t)__double2hiint(f);
+    if (farg + __ldg(tb.G + 1) > 60.0) { lo = 0u; hi = kInfHi; }       // floor dominates: beta uniform
+    if (farg + tabG(tb, n) < -104.0) { lo = 0u; hi = kNegInfHi; }      // floor negligible over the run
+    const float inv = hi == kInfHi ? 0.f : rcp_approx(sw);
+#pragma unroll
+    for (uint32_t q = 0; q < LM / 4; ++q)
+        recW[q * 32] = make_float4(bv[4 * q] * inv, bv[4 * q + 1] * inv, bv[4 * q + 2] * inv, bv[4 * q + 3] * inv);
+    *recF = make_uint4(lo, hi, pk, em);
 }
 
 // Backward records of window w (anchors [wC, min(wC + C, NA))) of one sample,
@@ -933,11 +976,12 @@ __device__ __forceinline__ void rebuild_window(const TypedArgs& A, const Tabs& t
     cp_async_wait_all();
     const uint32_t C = A.C;
     const uint32_t k0 = w * C, k1 = min(k0 + C, NA);
-    auto P = [&](uint32_t k) { return st.P[(k - k0) * 32 + lane]; };
-    auto E = [&](uint32_t k) { return st.E[(k - k0) * 32 + lane]; };
+    const uint32_t* P = st.P + lane;  // entry k at 32 (k - k0)
+    const uint32_t* E = st.E + lane;
+    recW += lane;
+    recF += lane;
     float bv[LM];
     double logU;
-    uint32_t kstart;
     if (k1 < NA) {
 #pragma unroll
         for (uint32_t q = 0; q < Q4; ++q) {
@@ -945,40 +989,71 @@ __device__ __forceinline__ void rebuild_window(const TypedArgs& A, const Tabs& t
             bv[4 * q] = x.x; bv[4 * q + 1] = x.y; bv[4 * q + 2] = x.z; bv[4 * q + 3] = x.w;
         }
         logU = st.U[lane];
-        kstart = k1;
-    } else {
+    }
+    if (C == 2 && k1 < NA) {  // the default window, without loops
+        const uint32_t pa = P[0], pb = P[32], pc = P[64] & ~kShiftBit, eb = E[32];
+        const uint32_t qb = pb & ~kShiftBit;
+        write_record<LM>(tb, pc - qb, bv, logU, pc, E[64], recW + Q4 * 32, recF + 32);
+        backward_step<LM>(tb, pc - qb, bv, logU, eb, pb >> 31);
+        write_record<LM>(tb, qb - (pa & ~kShiftBit), bv, logU, qb, eb, recW, recF);
+        return;
+    }
+    uint32_t r = k1 - k0;  // records left
+    if (k1 == NA) {
         // the chain's last run: beta is uniform there
-        const uint32_t pl = P(NA - 1);
+        const uint32_t pl = P[32 * (r - 1)];
         logU = chain_end_logU(tb, len - 1 - (pl & ~kShiftBit)) - ((pl & kShiftBit) ? 999.0 : 0.0);
-        init_forward<LM>(bv, E(NA - 1));
-        kstart = NA - 1;
-        const uint32_t r = NA - 1 - k0;
+        init_forward<LM>(bv, E[32 * (r - 1)]);
+        --r;
 #pragma unroll
-        for (uint32_t q = 0; q < Q4; ++q) recW[(r * Q4 + q) * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-        recF[r * 32 + lane] = make_uint4(0u, kInfHi, len, 0u);
+        for (uint32_t q = 0; q < Q4; ++q) recW[(r * Q4 + q) * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
+        recF[r * 32] = make_uint4(0u, kInfHi, len, 0u);
     }
-    for (uint32_t k = kstart; k > k0; --k) {
-        const uint32_t pk = P(k) & ~kShiftBit, pb = P(k - 1);
+    for (; r; --r) {
+        const uint32_t pk = P[32 * r] & ~kShiftBit, pb = P[32 * (r - 1)];
         const uint32_t n = pk - (pb & ~kShiftBit);
-        const float sw = vsum<LM>(bv);
-        const double farg = -999.0 - logU;
-        uint32_t lo = 0u, hi;
-        if (farg + tabG(tb, n) < -104.0) hi = kNegInfHi;  // floor negligible over the run
-        else if (farg + tabG(tb, 1) > 60.0) hi = kInfHi;  // floor dominates: beta uniform
-        else {
-            const double f = farg - (double)logf(sw);
-            lo = (uint32_t)__double_as_longlong(f);
-            hi = (uint32_t)((unsigned long long)__double_as_longlong(f) >> 32);
-        }
-        const uint32_t r = k - 1 - k0;
-        const float inv = hi == kInfHi ? 0.f : rcp_approx(sw);
-#pragma unroll
-        for (uint32_t q = 0; q < Q4; ++q)
-            recW[(r * Q4 + q) * 32 + lane] =
-                make_float4(bv[4 * q] * inv, bv[4 * q + 1] * inv, bv[4 * q + 2] * inv, bv[4 * q + 3] * inv);
-        recF[r * 32 + lane] = make_uint4(lo, hi, pk, E(k));
-        if (k - 1 > k0) backward_step<LM>(tb, n, bv, logU, E(k - 1), pb >> 31, 0u);
+        write_record<LM>(tb, n, bv, logU, pk, E[32 * r], recW + (r - 1) * Q4 * 32, recF + (r - 1) * 32);
+        if (r > 1) backward_step<LM>(tb, n, bv, logU, E[32 * (r - 1)], pb >> 31);
     }
+}
+
+// Barrier of the CTA's first n threads (whole warps), and whether x holds in all of them.
+__device__ __forceinline__ void cta_barrier(uint32_t n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
+__device__ __forceinline__ bool cta_all(bool x, uint32_t n) {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(r)
+                 : "r"((uint32_t)x), "r"(n)
+                 : "memory");
+    return r != 0;
+}
+
+// Whether every lane's sample has the lane 0 sample's region, length and anchor
+// count, and its anchor positions from k0 to the group's end k1.
+template <bool kPlain>
+__device__ __forceinline__ bool lanes_in_step(const TypedArgs& A, const View& v, uint32_t NA, uint32_t len, bool live,
+                                              const uint32_t* apos, uint32_t k0, uint32_t k1) {
+    constexpr uint32_t kAll = 0xffffffffu;
+    const uint32_t NA0 = __shfl_sync(kAll, NA, 0);
+    bool same = live && NA == NA0;
+    if (!kPlain) {
+        auto equal = [&](unsigned long long x) { return x == __shfl_sync(kAll, x, 0); };
+        same = equal(reinterpret_cast<unsigned long long>(v.r.masks)) && same;
+        same = equal(reinterpret_cast<unsigned long long>(v.r.tabs.QS)) && same;
+        same = equal((unsigned long long)len << 32 | v.r.L) && same;
+    }
+    if (!__all_sync(kAll, same)) return false;
+    k0 = __shfl_sync(kAll, k0, 0);
+    k1 = min(__shfl_sync(kAll, k1, 0), NA0 - 1);
+    for (uint32_t k = k0; k <= k1; k += 8) {
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t p = apos[32ull * min(k + j, k1)];
+            same = ((p ^ __shfl_sync(kAll, p, 0)) & ~kShiftBit) == 0u && same;
+        }
+        if (!__all_sync(kAll, same)) return false;
+    }
+    return true;
 }
 
 // kFull: every sample of the launch uses all LM slots (no active-slot masking).
@@ -989,10 +1064,8 @@ __device__ __forceinline__ void rebuild_window(const TypedArgs& A, const Tabs& t
 // A lane takes two consecutive cells of a run per step (an even marker and
 // the next one) with f32x2 arithmetic across the two cells; a run's odd first
 // marker or last marker takes a step alone (the second half is discarded).
-// The next step's run coefficients are loaded while the current step runs.
 // Tiles are aligned to absolute 32-marker columns, so a tile every lane of a
-// warp fills completely (lanes that share typed positions) leaves as 128-bit
-// row segments.
+// warp fills completely leaves as 128-bit row segments.
 template <int LM, bool kFull, bool kFast, bool kPlain, bool kDos>
 __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     anchor_posterior_kernel(const __grid_constant__ TypedArgs A) {
@@ -1000,13 +1073,14 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     constexpr uint32_t Q4 = LM / 4;
     constexpr uint32_t kAll = 0xffffffffu;
     constexpr bool kBcast = LM <= 16;  // a', w' held as (x, x) pairs: no per-step pairing moves
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    uint32_t lane;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));  // kept in a register, not read again at each use
+    const uint32_t warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const uint32_t C = A.C, K = A.K;
-    unsigned char* wbase = smem + (size_t)warp * post_warp_bytes(LM, C, !kFast);
+    unsigned char* wbase = smem + (A.stage ? post_cta_bytes(LM, kDos) : 0) + (size_t)warp * post_warp_bytes(LM, C, !kFast);
     float4* recW = reinterpret_cast<float4*>(wbase);                     // [C][Q4][32]
     uint4* recF = reinterpret_cast<uint4*>(recW + (size_t)C * Q4 * 32);  // [C][32]
-    uint4* meta = recF + (size_t)C * 32;                                 // [2][32]
-    float* tD = reinterpret_cast<float*>(meta + 64);                     // [32][36]
+    float* tD = reinterpret_cast<float*>(recF + (size_t)C * 32);         // [32][36]
     uint8_t* tH = reinterpret_cast<uint8_t*>(tD + 32 * 36);              // [64][36]
     float2* tP = reinterpret_cast<float2*>(tH + 64 * 36);                // [32][34] (P(hap=1) only)
     Staging st;
@@ -1015,24 +1089,25 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     st.P = reinterpret_cast<uint32_t*>(st.U + 32);
     st.E = st.P + (C + 1) * 32;
 
-    const uint32_t SG = (A.B + 31) / 32;
-    const unsigned long long gw = (unsigned long long)blockIdx.x * nw + warp;
-    const uint32_t g = (uint32_t)(gw % SG);
-    const uint32_t s = g * 32 + lane;
-    const unsigned long long grp = gw / SG;
-    bool live = s < A.B && grp * K < A.max_windows;
+    const uint32_t SG = (A.B + 31) / 32, SC = (SG + nw - 1) / nw;  // sample groups, CTAs of one window group
+    const unsigned long long grp = blockIdx.x / SC;
+    const uint32_t g0 = blockIdx.x % SC * nw, g = g0 + warp;
+    const uint32_t cta_threads = 32 * min(nw, SG - g0);  // the warps with samples
+    if (g >= SG) return;  // whole warp
+    // a lane past the batch's end repeats its last sample, and writes nothing
+    const bool real = g * 32 + lane < A.B;
+    const uint32_t s = real ? g * 32 + lane : A.B - 1;
+    bool live = grp * K < A.max_windows;
     View v{};
-    uint32_t NA = 0;
-    if (live) {
-        if (!kPlain) v = view_of(A, s);
-        NA = A.counts[s];
-    }
-    const unsigned long long ab = A.aoff[g] + lane, wb = A.woff[g] + lane;
+    if (!kPlain) v = view_of(A, s);
+    const uint32_t NA = A.counts[s];
+    const unsigned long long ab = A.aoff[g] + (s & 31u), wb = A.woff[g] + (s & 31u);
     const uint32_t NW = (NA + C - 1) / C;
     const uint32_t w0 = live ? (uint32_t)grp * K : 0u;
     const uint32_t wend = min(w0 + K, NW);
     live = live && w0 < wend;
-    if (!__any_sync(kAll, live)) return;  // whole warp
+    const bool warp_live = __any_sync(kAll, live);
+    if (!A.stage && !warp_live) return;  // whole warp
 
     const TypedRegion& R = kPlain ? A.reg0 : v.r;
     const uint32_t len = kPlain ? A.M : v.len;
@@ -1060,7 +1135,7 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     auto set_w = [&](int l, float x) { if constexpr (kBcast) w2[l] = make_float2(x, x); else wp[l] = x; };
     uint4 fr = make_uint4(0u, kNegInfHi, 0u, 0u);  // the current run's record: farg' lo, hi, end, end emission
     float2 FH = make_float2(0.f, 0.f), FL = make_float2(0.f, 0.f);  // a floor run's farg' as float hi + lo
-    uint32_t k = w0 * C, p0 = 0, p1 = 0, m = 0, mend = 0;
+    uint32_t p0 = 0, p1 = 0, m = 0, mend = 0;
     auto load_record = [&](uint32_t r) {
 #pragma unroll
         for (uint32_t q = 0; q < Q4; ++q) {
@@ -1087,7 +1162,7 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
         const float inv = rcp_approx(vsum<LM>(x));
 #pragma unroll
         for (int l = 0; l < LM; ++l) set_a(l, x[l] * inv);
-        p0 = apos[32ull * k] & ~kShiftBit;
+        p0 = apos[32ull * w0 * C] & ~kShiftBit;
         mend = wend * C < NA ? (apos[32ull * wend * C] & ~kShiftBit) : len;
         m = p0;
         rebuild_window<LM>(A, tb, NA, len, w0, st, recW, recF, lane);
@@ -1104,45 +1179,39 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     // filled columns [tlo, thi).
     auto flush = [&](uint32_t tbase, uint32_t tlo, uint32_t thi, bool on) {
         __syncwarp();
-        const bool has = on && thi > tlo;
+        const bool has = on && real && thi > tlo;
         const uint32_t tb0 = __shfl_sync(kAll, tbase, 0);
         if (__all_sync(kAll, vec_ok && has && tlo == 0 && thi == 32 && tbase == tb0)) {
             // every lane filled the same whole tile: 128-bit rows of dosage, 32-bit rows of alleles
             const unsigned long long s0 = s - lane;
+            const uint32_t r = lane >> 3, c = (lane & 7) * 4;  // four rows at a time
             if (w_dos) {
-#pragma unroll 4
-                for (uint32_t it = 0; it < 8; ++it) {
-                    const uint32_t r = it * 4 + (lane >> 3), c = (lane & 7) * 4;
-                    const float4 x = *reinterpret_cast<const float4*>(tD + r * 36 + c);
-                    *reinterpret_cast<float4*>(A.dosage + (s0 + r) * A.M + tb0 + c) = x;
-                }
+                float* to = A.dosage + (s0 + r) * A.M + tb0 + c;
+                const float* from = tD + r * 36 + c;
+#pragma unroll
+                for (uint32_t it = 0; it < 8; ++it, to += 4ull * A.M)
+                    *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(from + it * 4 * 36);
             }
-            if (w_hap) {
-#pragma unroll 4
-                for (uint32_t it = 0; it < 16; ++it) {
-                    const uint32_t rr = it * 4 + (lane >> 3), c = (lane & 7) * 4;
-                    const uint32_t x = *reinterpret_cast<const uint32_t*>(tH + rr * 36 + c);
-                    *reinterpret_cast<uint32_t*>(A.haps + (2 * (s0 + (rr >> 1)) + (rr & 1)) * A.M + tb0 + c) = x;
-                }
+            if (w_hap) {  // rows 2 s, 2 s + 1 follow each other
+                uint8_t* to = A.haps + (2 * s0 + r) * A.M + tb0 + c;
+                const uint8_t* from = tH + r * 36 + c;
+#pragma unroll
+                for (uint32_t it = 0; it < 16; ++it, to += 4ull * A.M)
+                    *reinterpret_cast<uint32_t*>(to) = *reinterpret_cast<const uint32_t*>(from + it * 4 * 36);
             }
         } else {
-            const unsigned long long od = out + tbase, oh = 2ull * out + tbase;
-            meta[lane] = make_uint4((uint32_t)od, (uint32_t)(od >> 32), (uint32_t)oh, (uint32_t)(oh >> 32));
-            meta[32 + lane] = make_uint4(len, tlo, thi, has ? 1u : 0u);
-            __syncwarp();
             for (uint32_t r = 0; r < 32; ++r) {
-                const uint4 m1 = meta[32 + r];
-                if (!m1.w) continue;  // same value in every lane
-                const uint4 m0 = meta[r];
-                if (lane >= m1.y && lane < m1.z) {
-                    const unsigned long long rd = ((unsigned long long)m0.y << 32) | m0.x;
-                    const unsigned long long rh = ((unsigned long long)m0.w << 32) | m0.z;
-                    if (w_dos) A.dosage[rd + lane] = tD[r * 36 + lane];
+                if (!__shfl_sync(kAll, has, r)) continue;
+                const unsigned long long ro = __shfl_sync(kAll, out, r);
+                const uint32_t rl = __shfl_sync(kAll, len, r), at = __shfl_sync(kAll, tbase, r) + lane;
+                const uint32_t lo = __shfl_sync(kAll, tlo, r), hi = __shfl_sync(kAll, thi, r);
+                if (lane >= lo && lane < hi) {
+                    if (w_dos) A.dosage[ro + at] = tD[r * 36 + lane];
                     if (w_hap) {
-                        A.haps[rh + lane] = tH[(2 * r) * 36 + lane];
-                        A.haps[rh + m1.x + lane] = tH[(2 * r + 1) * 36 + lane];
+                        A.haps[2 * ro + at] = tH[(2 * r) * 36 + lane];
+                        A.haps[2 * ro + rl + at] = tH[(2 * r + 1) * 36 + lane];
                     }
-                    if (w_hp) reinterpret_cast<float2*>(A.hprob)[rd + lane] = tP[r * 34 + lane];
+                    if (w_hp) reinterpret_cast<float2*>(A.hprob)[ro + at] = tP[r * 34 + lane];
                 }
             }
         }
@@ -1153,8 +1222,8 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     auto coeffs = [&](uint32_t mm, float4& qa, float4& qb) {
         const uint32_t i = mm - p0, j = p1 - mm;
         if (in_tab) {
-            qa = __ldg(tb.QSup + i);
-            qb = __ldg(tb.QSdn + j);
+            qa = __ldg(tb.up + i);
+            qb = __ldg(tb.dg + 2 * j);
         } else {
             const float2 x0 = tabQS(tb, i), x1 = tabQS(tb, i + 1), y0 = tabQS(tb, j), y1 = tabQS(tb, j - 1);
             qa = make_float4(x0.x, x1.x, x0.y, x1.y);
@@ -1174,7 +1243,7 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
             if (in_tab) {
                 // (hi + hi) + (lo + lo) in FP32: where the floor is within reach of the carried
                 // terms the high parts nearly cancel, and their sum is exact
-                const float4 g = __ldg(tb.Gdn + j);
+                const float4 g = __ldg(tb.dg + 2 * j + 1);
                 ft2 = __fadd2_rn(__fadd2_rn(FH, make_float2(g.x, g.y)), __fadd2_rn(FL, make_float2(g.z, g.w)));
             } else {
                 const double fa = __hiloint2double((int)fr.y, (int)fr.x);
@@ -1280,6 +1349,258 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
         }
     };
 
+    // the next anchor: alpha steps over the current run and takes its emission, and the run starting
+    // there becomes the current one
+    uint32_t rec = 0, win = w0;  // the current run's record, its window
+    auto anchor = [&](float2 qs) {
+        const uint32_t em = fr.w;
+        if (++rec == C) {
+            rec = 0;
+            ++win;
+            rebuild_window<LM>(A, tb, NA, len, win, st, recW, recF, lane);
+            if (win + 1 < wend) stage_window<LM>(A, apos, aem, wb, NA, win + 1, st, lane);
+        }
+        float x[LM];
+#pragma unroll
+        for (int l = 0; l < LM; ++l) x[l] = a_of(l);
+        const float base = vsum<LM>(x) * qs.y;
+#pragma unroll
+        for (int l = 0; l < LM; ++l) x[l] = ((em >> l) & 1u) ? fmaf(qs.x, x[l], base) : 0.f;
+        const float inv = rcp_approx(vsum<LM>(x));
+#pragma unroll
+        for (int l = 0; l < LM; ++l) set_a(l, x[l] * inv);
+        load_record(rec);
+    };
+
+    // ---- lanes in step: every lane's sample has the same anchors (an array's sites). All control and
+    // every address but the outputs' is then the warp's own, not a lane's.
+    const bool in_step = warp_live && lanes_in_step<kPlain>(A, v, NA, len, live, apos, w0 * C, wend * C);
+    // The warps of a CTA walk the same window group of neighbouring samples. If they are all in step, the CTA
+    // keeps the markers' slot data and the head of the run tables in shared memory, a tile ahead: read from
+    // global memory they missed L1 (28 KB beside this kernel's shared memory) two times out of three.
+    bool staged = false;
+    float4* sT = reinterpret_cast<float4*>(smem);                    // [kPostTab] up, [kPostTab][2] dg
+    SlotMasks* sM = reinterpret_cast<SlotMasks*>(sT + 3 * kPostTab);  // [2][32]
+    float4* sG = reinterpret_cast<float4*>(sM + 64);                 // [2][32][gs / 2]
+    if (A.stage) {
+        unsigned long long* what = reinterpret_cast<unsigned long long*>(smem + post_cta_bytes(LM, kDos) - 32);
+        const unsigned long long mine[4] = {(unsigned long long)m << 32 | mend,
+                                            reinterpret_cast<unsigned long long>(R.masks),
+                                            reinterpret_cast<unsigned long long>(tb.QS), R.gs};
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) what[i] = mine[i];
+        }
+        cta_barrier(cta_threads);
+        bool same = in_step;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) same = same && what[i] == mine[i];
+        staged = cta_all(same, cta_threads);
+        if (!warp_live) return;  // whole warp, of a CTA that does not stage
+    }
+    if (staged) {
+        auto warp_value = [&](uint32_t x) { return __reduce_max_sync(kAll, x); };
+        uint32_t um = warp_value(m), u0 = um, u1 = warp_value(p1);
+        const uint32_t uend = warp_value(mend);
+        const uint32_t rows = min(32u, A.B - g * 32);
+        // the current run's floor on one form for every lane, so that a step needs no branch: -3e38
+        // stands for a negligible floor (F = 0), 3e38 for a uniform run (X w' = 0 there, Y F + 1 = 1)
+        auto one_form = [&] {
+            if ((fr.y & kInfHi) == kInfHi) {
+                const float h = fr.y == kInfHi ? 3e38f : -3e38f;
+                FH = make_float2(h, h);
+                FL = make_float2(0.f, 0.f);
+            }
+        };
+        one_form();
+        const float4* g2 = reinterpret_cast<const float4*>(R.g2);
+        const uint32_t gq = kPlain ? LM / 2 : R.gs / 2;  // float4s of a marker's weights
+        const bool has_raw = R.raw != nullptr;
+        const SlotMasks* mrow = sM;  // the current tile's slot data
+        const float4* grow = sG;
+        float* const tDl = tD + lane * 36;
+        uint8_t* const tHl = tH + 2 * lane * 36;
+        auto stage_tile = [&](uint32_t t0, uint32_t b) {  // slot data of markers [t0, t0 + 32)
+            if (t0 >= uend) return;
+            const uint32_t nm = min(32u, len - t0);
+            for (uint32_t x = threadIdx.x; x < nm; x += cta_threads) cp_async16(sM + 32 * b + x, R.masks + t0 + x);
+            if constexpr (post_stage_weights(LM, kDos))
+                for (uint32_t x = threadIdx.x; x < nm * gq; x += cta_threads)
+                    cp_async16(sG + 32 * gq * b + x, g2 + (size_t)t0 * gq + x);
+        };
+        for (uint32_t x = threadIdx.x; x < 3 * kPostTab; x += cta_threads)
+            cp_async16(sT + x, x < kPostTab ? tb.up + x : tb.dg + (x - kPostTab));
+        stage_tile(um & ~31u, 0);
+        // cells mm and mm + 1 (the second one discarded unless two) into columns c0, c0 + 1
+        auto pair = [&](uint32_t mm, auto two, const float4* pu, const float4* pd, uint32_t c0) {
+            const float4 qa = *pu, qb = pd[0], gv = pd[1];
+            const SlotMasks mkA = mrow[c0];
+            const SlotMasks mkB = two ? mrow[c0 + 1] : mkA;
+            float2 XX = make_float2(qb.x, qb.y), YY = make_float2(qb.z, qb.w);
+            // floor e^ft beside X w' + Y; when it dominates (ft > 0) both are scaled by e^-ft. e^-|ft| below the
+            // smallest normal number reads 0: it is added to 1 or to Y >= 1e-30, which it would not change.
+            const float2 ft = __fadd2_rn(__fadd2_rn(FH, make_float2(gv.x, gv.y)), __fadd2_rn(FL, make_float2(gv.z, gv.w)));
+            const float e0 = ex2_ftz(fabsf(ft.x) * -1.44269504088896341f), e1 = ex2_ftz(fabsf(ft.y) * -1.44269504088896341f);
+            const bool big0 = ft.x > 0.f, big1 = ft.y > 0.f;
+            const float2 xs = make_float2(big0 ? e0 : 1.f, big1 ? e1 : 1.f);
+            YY = __ffma2_rn(YY, xs, make_float2(big0 ? 1.f : e0, big1 ? 1.f : e1));
+            XX = __fmul2_rn(XX, xs);
+            const float2 QQ = make_float2(qa.x, qa.y), SS = make_float2(qa.z, qa.w);
+            float2 p2[LM];
+#pragma unroll
+            for (int l = 0; l < LM; ++l) {
+                p2[l] = __fmul2_rn(__ffma2_rn(QQ, A2(l), SS), __ffma2_rn(XX, W2(l), YY));
+                if (!kFull && (uint32_t)l >= Lr) p2[l] = make_float2(0.f, 0.f);
+            }
+            float2 inv2 = make_float2(0.f, 0.f);
+            float2 tot2 = inv2;
+            if (kDos || !kFast) {
+                float2 t2[LM / 2];
+#pragma unroll
+                for (int l = 0; l < LM / 2; ++l) t2[l] = __fadd2_rn(p2[2 * l], p2[2 * l + 1]);
+#pragma unroll
+                for (int h = LM / 4; h >= 1; h >>= 1)
+#pragma unroll
+                    for (int l = 0; l < h; ++l) t2[l] = __fadd2_rn(t2[l], t2[l + h]);
+                tot2 = t2[0];
+                inv2 = make_float2(rcp_approx(tot2.x), rcp_approx(tot2.y));
+            }
+            if constexpr (kDos) {
+                float2 d2 = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int q = 0; q < LM / 2; ++q) {
+                    if (kFull || (uint32_t)(2 * q) < 2 * gq) {
+                        float4 w;
+                        if constexpr (post_stage_weights(LM, kDos)) w = grow[c0 * gq + q];
+                        else w = __ldg(g2 + (size_t)mm * gq + q);
+                        d2 = __ffma2_rn(p2[2 * q], make_float2(w.x, w.y), d2);
+                        d2 = __ffma2_rn(p2[2 * q + 1], make_float2(w.z, w.w), d2);
+                    }
+                }
+                const float2 dos2 = __fmul2_rn(d2, inv2);
+                if (two) *reinterpret_cast<float2*>(tDl + c0) = dos2;
+                else tDl[c0] = dos2.x;
+            }
+            uint32_t pk[2];
+            if (argmax) {
+                pick_pair<LM>(p2, keep, pk[0], pk[1]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const float target = cell_uniform(A.seed, kPlain ? A.sid_base + s : v.sid,
+                                                      (kPlain ? 0u : v.m0) + mm + c) * (c ? tot2.y : tot2.x);
+                    float cum = 0.f;
+                    uint32_t last_nz = 0, pick = LM;
+#pragma unroll
+                    for (int l = 0; l < LM; ++l) {
+                        const float pl = c ? p2[l].y : p2[l].x;
+                        cum += pl;
+                        if (pl > 0.f) last_nz = (uint32_t)l;
+                        if (pick == LM && target < cum) pick = (uint32_t)l;
+                    }
+                    pk[c] = pick == LM ? last_nz : pick;
+                }
+            }
+            // the picks' alleles: bytes {hap0 A, hap0 B, hap1 A, hap1 B}
+            uint32_t hv;
+            if (has_raw && (mkA.x | mkB.x) != 0u) {
+                const uint32_t hA = slot_alleles(mkA, R.raw, R.gs, mm, pk[0]);
+                const uint32_t hB = two ? slot_alleles(mkB, R.raw, R.gs, mm + 1, pk[1]) : 0u;
+                hv = (hA & 0xffu) | (hB & 0xffu) << 8 | (hA >> 8) << 16 | (hB >> 8) << 24;
+            } else if constexpr (LM <= 16) {
+                hv = (shr(mkA.a0 | mkA.a1 << 16, pk[0]) & 0x10001u) + (shr(mkB.a0 | mkB.a1 << 16, pk[1]) & 0x10001u) * 256u;
+            } else {
+                hv = (shr(mkA.a0, pk[0]) & 1u) | (shr(mkB.a0, pk[1]) & 1u) << 8 | (shr(mkA.a1, pk[0]) & 1u) << 16 |
+                     (shr(mkB.a1, pk[1]) & 1u) << 24;
+            }
+            if (two) {
+                *reinterpret_cast<uint16_t*>(tHl + c0) = (uint16_t)hv;
+                *reinterpret_cast<uint16_t*>(tHl + 36 + c0) = (uint16_t)(hv >> 16);
+            } else {
+                tHl[c0] = (uint8_t)hv;
+                tHl[36 + c0] = (uint8_t)(hv >> 16);
+            }
+            if (w_hp) {
+                float q0[2] = {0.f, 0.f}, q1[2] = {0.f, 0.f};
+#pragma unroll
+                for (int l = 0; l < LM; ++l) {
+                    q0[0] += ((mkA.a0 >> l) & 1u) ? p2[l].x : 0.f;
+                    q1[0] += ((mkA.a1 >> l) & 1u) ? p2[l].x : 0.f;
+                    q0[1] += ((mkB.a0 >> l) & 1u) ? p2[l].y : 0.f;
+                    q1[1] += ((mkB.a1 >> l) & 1u) ? p2[l].y : 0.f;
+                }
+                if (two)
+                    *reinterpret_cast<float4*>(tP + lane * 34 + c0) =
+                        make_float4(q0[0] * inv2.x, q1[0] * inv2.x, q0[1] * inv2.y, q1[1] * inv2.y);
+                else tP[lane * 34 + c0] = make_float2(q0[0] * inv2.x, q1[0] * inv2.x);
+            }
+        };
+        uint32_t buf = 0;
+        for (uint32_t utb = um & ~31u; um < uend; utb += 32, buf ^= 1u) {
+            const uint32_t lo = um - utb, tend = min(utb + 32, uend);
+            cp_async_wait_all();
+            cta_barrier(cta_threads);  // this tile's slot data are there; the last tile's have been read
+            stage_tile(utb + 32, buf ^ 1u);
+            mrow = sM + 32 * buf;
+            grow = sG + 32 * gq * buf;
+            while (um < tend) {
+                if (um == u1) {
+                    anchor(tabQS(tb, u1 - u0));
+                    u0 = u1;
+                    u1 = warp_value(fr.z);
+                    p0 = u0;
+                    p1 = u1;
+                    in_tab = u1 - u0 < tb.NT;
+                    one_form();
+                }
+                const uint32_t e = min(u1, tend);
+                if (u1 - u0 < tb.NT) {
+                    const bool head = u1 - u0 < kPostTab;
+                    const float4* pu = (head ? sT : tb.up) + (um - u0);
+                    const float4* pd = (head ? sT + kPostTab : tb.dg) + 2 * (u1 - um);
+                    if (um & 1u) {
+                        pair(um, std::false_type{}, pu, pd, um - utb);
+                        ++um, ++pu, pd -= 2;
+                    }
+                    for (; um + 1 < e; um += 2, pu += 2, pd -= 4) pair(um, std::true_type{}, pu, pd, um - utb);
+                    if (um < e) {
+                        pair(um, std::false_type{}, pu, pd, um - utb);
+                        ++um;
+                    }
+                } else {  // a run longer than the tables
+                    for (; um < e; ++um) {
+                        float4 qa, qb;
+                        coeffs(um, qa, qb);
+                        cells(um, false, qa, qb, um - utb);
+                    }
+                }
+            }
+            if (vec_ok && lo == 0 && tend == utb + 32 && rows == 32) {
+                flush(utb, 0, 32, true);
+            } else {  // rows at any offset, one 32-marker segment after the other
+                __syncwarp();
+                const bool col = lane >= lo && utb + lane < tend;
+                const unsigned long long od = out + utb + lane;
+#pragma unroll 4
+                for (uint32_t r = 0; r < rows; ++r) {
+                    const unsigned long long rd = kPlain ? (unsigned long long)(g * 32 + r) * A.M + utb + lane
+                                                         : __shfl_sync(kAll, od, r) - r + lane;
+                    if (col) {
+                        if (w_dos) A.dosage[rd] = tD[r * 36 + lane];
+                        if (w_hp) reinterpret_cast<float2*>(A.hprob)[rd] = tP[r * 34 + lane];
+                        if (w_hap) {
+                            const unsigned long long rh = 2 * rd - utb - lane;  // 2 x the row's offset + the marker
+                            A.haps[rh] = tH[(2 * r) * 36 + lane];
+                            A.haps[rh + len] = tH[(2 * r + 1) * 36 + lane];
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        return;
+    }
+
     uint32_t tbase = m & ~31u;
     for (;;) {
         const bool on = live && m < mend;
@@ -1290,25 +1611,7 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
             tlo = m - tbase;
             while (m < tend) {
                 if (m == p1) {
-                    // anchor k + 1: alpha steps over the run and takes its emission
-                    const uint32_t kn = k + 1, n = p1 - p0, em = fr.w;
-                    if (kn % C == 0) {
-                        const uint32_t wn = kn / C;
-                        rebuild_window<LM>(A, tb, NA, len, wn, st, recW, recF, lane);
-                        if (wn + 1 < wend) stage_window<LM>(A, apos, aem, wb, NA, wn + 1, st, lane);
-                    }
-                    const float2 qs = tabQS(tb, n);
-                    float x[LM];
-#pragma unroll
-                    for (int l = 0; l < LM; ++l) x[l] = a_of(l);
-                    const float base = vsum<LM>(x) * qs.y;
-#pragma unroll
-                    for (int l = 0; l < LM; ++l) x[l] = ((em >> l) & 1u) ? fmaf(qs.x, x[l], base) : 0.f;
-                    const float inv = rcp_approx(vsum<LM>(x));
-#pragma unroll
-                    for (int l = 0; l < LM; ++l) set_a(l, x[l] * inv);
-                    load_record(kn % C);
-                    k = kn;
+                    anchor(tabQS(tb, p1 - p0));
                     p0 = p1;
                     p1 = fr.z;
                     in_tab = p1 - p0 < tb.NT;
@@ -1338,7 +1641,11 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
 template <int LM, bool kFull, bool kFast, bool kPlain, bool kDos = true>
 cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
     const uint32_t T = a.threads;
-    const size_t sm = (size_t)(T / 32) * post_warp_bytes(LM, a.C, !kFast);
+    // the CTA's part is left out where it would not fit beside the windows
+    size_t sm = (size_t)(T / 32) * post_warp_bytes(LM, a.C, !kFast);
+    TypedArgs f = a;
+    f.stage = sm + post_cta_bytes(LM, kDos) <= 227u * 1024u;
+    if (f.stage) sm += post_cta_bytes(LM, kDos);
     // set outside stream capture only (a plan launches once before it is captured)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &cs);
@@ -1349,11 +1656,10 @@ cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
         if (e != cudaSuccess) return e;
     }
     const unsigned long long groups = ((unsigned long long)a.max_windows + a.K - 1) / a.K;
-    const unsigned long long warps = (unsigned long long)((a.B + 31) / 32) * groups;
-    const unsigned long long grid = (warps + T / 32 - 1) / (T / 32);
+    const unsigned long long grid = groups * ((typed_groups(a.B) + T / 32 - 1) / (T / 32));
     if (grid == 0) return cudaSuccess;
     if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-    anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos><<<(uint32_t)grid, T, sm, s>>>(a);
+    anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos><<<(uint32_t)grid, T, sm, s>>>(f);
     return cudaGetLastError();
 }
 
@@ -1388,7 +1694,7 @@ uint32_t typed_default_window(uint32_t) { return 2u; }
 uint32_t typed_default_threads(uint32_t lmax) { return lmax <= 16 ? 128u : 64u; }
 
 size_t typed_post_smem_bytes(uint32_t L, uint32_t T, uint32_t C) {
-    return (size_t)(T / 32) * post_warp_bytes(fb_lmax(L), C, true);
+    return (size_t)(T / 32) * (post_warp_bytes(fb_lmax(L), C, true) + 1024);  // 1 KB a warp kept free
 }
 
 cudaError_t launch_anchor_count_only(const TypedArgs& a, cudaStream_t s) {

@@ -80,3 +80,33 @@ def test_list_rows(engine, M):
     codes[2, -1] = codes_all[2, -1]
     codes[3] = np.where(codes[3] == 3, rng.integers(3, 256, M), codes[3])  # any byte above 2 is a missing call
     check(engine, panel, pos, codes, 8)
+
+
+# targets of one array (the lanes of a CTA in step, slot data staged) against the same targets beside
+# others with sites of their own (each lane by itself): bit for bit the same, and the oracle's. Runs shorter
+# and longer than the staged head of the tables (64), one past the tables (4,096), odd rows, partial groups.
+@pytest.mark.parametrize("L,M,every,B,spacing", [(8, 333, 7, 33, 1000), (4, 1024, 64, 129, 1000), (3, 1000, 65, 31, 500_000),
+                                                 (16, 700, 63, 64, 1000), (32, 515, 130, 40, 1000),
+                                                 (8, 9001, 4500, 5, 1000), (8, 640, 1, 32, 500_000)])
+@pytest.mark.parametrize("other_alleles", [False, True])
+def test_posterior_walks(engine, L, M, every, B, spacing, other_alleles):
+    panel, pos, _ = synth.make_panel(M, 384, 20, seed=M + L, spacing=spacing)
+    codes, _, _ = synth.make_targets(panel, B, synth.typed_every(M, every), seed=M + 1, het_range=(0.0, 1.0))
+    if other_alleles:
+        u = np.random.default_rng(M).random(panel.shape)
+        panel = panel.copy()
+        panel[u < 0.02] = 255
+        panel[(u >= 0.02) & (u < 0.03)] = 2
+    check(engine, panel, pos, codes, L)
+    all_codes, _, _ = synth.make_targets((panel != 0).astype(np.uint8), B, np.arange(M), seed=M + 2, het_range=(0.0, 1.0))
+    mixed = np.empty((2 * B, M), np.uint8)
+    mixed[0::2] = codes
+    mixed[1::2] = own_sites(all_codes, np.random.default_rng(M).integers(0, M // 2, B), seed=M + 3)
+    for kw in ({}, {"sampling": N.SAMPLE_PHILOX}):
+        for out in ({"hap_prob": True}, {}, {"dosage": False}):
+            p = N.default_params(num_states=L, ne=20000, **kw)
+            alone = engine.impute(codes, p, **out)
+            beside = engine.impute(mixed, p, **out)
+            for key in alone:
+                if key != "haps" or not kw:  # a draw is keyed by the row's sample id
+                    assert np.array_equal(alone[key], beside[key][0::2]), (key, kw, out)
