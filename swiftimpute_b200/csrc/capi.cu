@@ -24,11 +24,17 @@ si_status dev_alloc(si_ctx* ctx, DeviceBuffer& buf, size_t bytes) {
     dev_free(ctx, buf);
     if (bytes == 0) bytes = 16;
     bytes = (bytes + 255) & ~size_t(255);
+    if (ctx->used + bytes > ctx->budget) dev_free(ctx, ctx->bckpt);  // waits for the kernels that use it
     if (ctx->used + bytes > ctx->budget)
         return fail(ctx, SI_ERR_BUDGET, "HBM budget exceeded: need " + std::to_string(bytes) + " more bytes, " +
                                             std::to_string(ctx->budget - ctx->used) + " left");
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->bckpt.ptr) {
+        cudaGetLastError();
+        dev_free(ctx, ctx->bckpt);
+        e = cudaMalloc(&p, bytes);
+    }
     if (e != cudaSuccess) { cudaGetLastError(); return cuda_fail(ctx, e, "cudaMalloc"); }
     buf.ptr = p;
     buf.bytes = bytes;
@@ -474,8 +480,30 @@ si_status run_device(si_ctx* ctx, const si_impute_params* p, const uint8_t* d_ge
         return fail(ctx, SI_ERR_UNSUPPORTED,
                     "tile (" + std::to_string(T) + " chains x " + std::to_string(C) + " markers) needs " +
                         std::to_string(fb_smem_bytes(p->num_states, T, C)) + " bytes of shared memory (max 227 KB)");
-    SI_TRY(dev_reserve(ctx, ctx->ckpt, fb_ckpt_bytes(B, ctx->M, p->num_states, C)));
     FbLaunch l;
+    l.ckpt = l.bckpt = nullptr;
+    // The segments run in parallel where both directions' ends find room, in half the default
+    // segment (half the alpha tile: twice the warps an SM) or else a whole one; a budget (or
+    // device) without room for either takes the one-pass kernel. The results are the same.
+    const uint32_t whole = C;
+    for (uint32_t c : {p->checkpoint_interval ? C : C / 2, C}) {
+        const size_t ends = (fb_ckpt_bytes(B, ctx->M, p->num_states, c) + 255) & ~size_t(255);
+        const size_t need = ends + fb_back_bytes(B, ctx->M, p->num_states, c);
+        if (ctx->bckpt.bytes < need) {
+            dev_free(ctx, ctx->bckpt);
+            if (ctx->used + need + 255 > ctx->budget) continue;
+            if (dev_alloc(ctx, ctx->bckpt, need) != SI_OK) continue;
+        }
+        C = c;
+        l.ckpt = (float*)ctx->bckpt.ptr;
+        l.bckpt = (float*)((char*)ctx->bckpt.ptr + ends);
+        break;
+    }
+    if (!l.bckpt) {
+        C = whole;
+        SI_TRY(dev_reserve(ctx, ctx->ckpt, fb_ckpt_bytes(B, ctx->M, p->num_states, C)));
+        l.ckpt = (float*)ctx->ckpt.ptr;
+    }
     l.geno = d_geno;
     l.masks = target ? nullptr : (const SlotMasks*)sel->masks.ptr;
     l.smasks = target ? (const SlotMasks*)ctx->smasks.ptr : nullptr;
@@ -483,7 +511,7 @@ si_status run_device(si_ctx* ctx, const si_impute_params* p, const uint8_t* d_ge
     l.trans = (const LinTrans*)ctx->trans.ptr;
     l.B = B; l.M = ctx->M; l.L = p->num_states; l.C = C; l.threads = T;
     l.sampling = p->sampling; l.tie_eps = (float)p->tie_eps; l.seed = p->seed; l.sample_id_base = p->sample_id_base;
-    l.ckpt = (float*)ctx->ckpt.ptr; l.dosage = d_dosage; l.hprob = d_hprob; l.haps = d_haps;
+    l.dosage = d_dosage; l.hprob = d_hprob; l.haps = d_haps;
     SI_CUDA(ctx, cudaEventRecord(ctx->ev[1], s), "event");
     SI_CUDA(ctx, cudaEventRecord(ctx->kev[2], s), "event");
     SI_CUDA(ctx, cudaEventRecord(ctx->kev[3], s), "event");
@@ -714,6 +742,7 @@ si_status si_ctx_destroy(si_ctx* ctx) {
     dev_free(ctx, ctx->panel);
     dev_free(ctx, ctx->trans);
     dev_free(ctx, ctx->ckpt);
+    dev_free(ctx, ctx->bckpt);
     dev_free(ctx, ctx->smasks);
     dev_free(ctx, ctx->io_geno);
     dev_free(ctx, ctx->io_dosage);
@@ -751,7 +780,7 @@ const char* si_last_error(const si_ctx* ctx) { return ctx ? ctx->err.c_str() : "
 
 si_status si_ctx_memory(const si_ctx* ctx, uint64_t* used_bytes, uint64_t* budget_bytes) {
     if (!ctx) return SI_ERR_INVALID_ARG;
-    if (used_bytes) *used_bytes = ctx->used;
+    if (used_bytes) *used_bytes = ctx->used - ctx->bckpt.bytes;  // bckpt makes room for any other allocation
     if (budget_bytes) *budget_bytes = ctx->budget;
     return SI_OK;
 }

@@ -109,6 +109,15 @@ extern "C" si_status si_impute_device_noalloc(si_ctx* ctx, const si_impute_param
     l.B = B; l.M = ctx->M; l.L = L; l.C = C; l.threads = T;
     l.sampling = p->sampling; l.tie_eps = (float)p->tie_eps; l.seed = p->seed; l.sample_id_base = p->sample_id_base;
     l.ckpt = (float*)scratch;
+    l.bckpt = nullptr;
+    // beta's ends behind alpha's, where the array has room for both (half the default segment first, as si_impute_device)
+    for (uint32_t c : {p->checkpoint_interval ? C : C / 2, C}) {
+        const size_t at = (fb_ckpt_bytes(B, ctx->M, L, c) + 255) & ~size_t(255);
+        if (at + fb_back_bytes(B, ctx->M, L, c) > kNoAllocScratchBytes) continue;
+        l.bckpt = (float*)((char*)scratch + at);
+        l.C = c;
+        break;
+    }
     l.dosage = d_dosage; l.hprob = d_hap_prob; l.haps = d_haps;
     e = launch_fb(l, stream ? (cudaStream_t)stream : ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "forward-backward kernel");

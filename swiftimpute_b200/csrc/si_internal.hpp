@@ -119,6 +119,7 @@ struct si_ctx {
     uint64_t trans_key = ~0ull;
     si::LinTrans trans0{1.f, 0.f};  // host copy of the first gap's transition
     si::DeviceBuffer ckpt;           // forward checkpoints (full-chain kernel)
+    si::DeviceBuffer bckpt;          // both directions' segment ends: held while the budget has room, freed for any other allocation
     si::DeviceBuffer smasks;         // per-target slot masks [M][B] (target-aware selection)
     // typed-marker kernel scratch and tables
     si::DeviceBuffer t_counts, t_segc, t_aoff, t_woff, t_apos, t_aem, t_ckF, t_ckB, t_ckU;
@@ -203,7 +204,8 @@ struct FbLaunch {
     int sampling;
     float tie_eps;
     uint64_t seed, sample_id_base;
-    float* ckpt;           // [B][nseg][Lmax]
+    float* ckpt;           // fb_ckpt_bytes of scratch: alpha at the segments' ends
+    float* bckpt;          // fb_back_bytes of scratch (8-byte aligned): beta at the segments' ends, or null
     float* dosage;         // [B][M] or null
     float* hprob;          // [B][M][2] or null
     uint8_t* haps;         // [B][2][M] or null
@@ -218,6 +220,7 @@ cudaError_t launch_target_select(const uint8_t* d_geno, uint32_t B, uint32_t M, 
                                  const uint32_t* d_prefix, const uint32_t* d_panel, const uint32_t* d_bits,
                                  const uint32_t* d_zeros, SlotMasks* d_smasks, uint32_t* d_pairs, cudaStream_t s);
 size_t fb_ckpt_bytes(uint32_t B, uint32_t M, uint32_t L, uint32_t C);
+size_t fb_back_bytes(uint32_t B, uint32_t M, uint32_t L, uint32_t C);
 // slots held per thread (and the stride of per-slot tables) for L slots
 inline __host__ __device__ uint32_t fb_lmax(uint32_t L) { return L <= 4 ? 4 : L <= 8 ? 8 : L <= 16 ? 16 : 32; }
 size_t fb_smem_bytes(uint32_t L, uint32_t T, uint32_t C);

@@ -110,3 +110,35 @@ def test_posterior_walks(engine, L, M, every, B, spacing, other_alleles):
             for key in alone:
                 if key != "haps" or not kw:  # a draw is keyed by the row's sample id
                     assert np.array_equal(alone[key], beside[key][0::2]), (key, kw, out)
+
+
+# the full chain in parallel segments against the oracle and against one pass over the chain (the
+# kernel that a budget without room for the segments' ends falls back to):
+# lengths around the checkpoint segments, the staged blocks (8, 4) and code chunks (32), B around a warp
+@pytest.mark.parametrize("L,M,B,C", [(8, 1, 3, 0), (8, 2, 33, 0), (8, 31, 5, 0), (8, 32, 31, 0), (8, 33, 32, 0),
+                                     (3, 65, 7, 0), (8, 500, 40, 7), (16, 257, 33, 0), (32, 131, 35, 0),
+                                     (32, 64, 3, 16), (4, 1000, 64, 1), (8, 1029, 130, 32)])
+@pytest.mark.parametrize("per_gap", [False, True])
+def test_full_chain_segments(engine, L, M, B, C, per_gap):
+    panel, pos, _ = synth.make_panel(M, 256, 20, seed=M + L, spacing=1000)
+    rng = np.random.default_rng(M)
+    pos = np.cumsum(rng.integers(1, 5000, M)).astype(np.uint64)
+    codes_all, _, _ = synth.make_targets(panel, B, np.arange(M), seed=M + 1, het_range=(0.0, 1.0))
+    codes = own_sites(codes_all, rng.integers(0, M + 1, B), seed=M + 2)
+    kw = {"flags": N.IMPUTE_FULL_CHAIN, "checkpoint_interval": C}
+    got = check(engine, panel, pos, codes, L, per_gap=per_gap, **kw)
+    # the same call in a context whose budget just holds what one pass needs
+    p = N.default_params(num_states=L, ne=20000, transition_mode=N.TRANS_PER_GAP if per_gap else N.TRANS_MATRIX0, **kw)
+    from swiftimpute_b200.engine import Engine
+    with Engine(0) as wide:
+        wide.upload_panel(panel); wide.set_map(pos); wide.pbwt_build()
+        wide.impute(codes, p, hap_prob=True)
+        used, _ = wide.memory()  # without the segments' ends, which make room for any other allocation
+    lmax = next(x for x in (4, 8, 16, 32) if L <= x)
+    c = C or (16 if lmax == 32 else 32)
+    one = (max(-(-M // c) - 1, 1) * lmax * B * 4 + 255) // 256 * 256  # the one pass' own checkpoints
+    with Engine(0, hbm_budget_bytes=max(used + one, 1 << 20)) as tight:
+        tight.upload_panel(panel); tight.set_map(pos); tight.pbwt_build()
+        one_pass = tight.impute(codes, p, hap_prob=True)
+    for key in got:
+        assert np.array_equal(got[key], one_pass[key]), key
