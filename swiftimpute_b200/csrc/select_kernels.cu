@@ -162,45 +162,143 @@ __global__ void target_rank_kernel(const uint32_t* __restrict__ prefix, const ui
     }
 }
 
-// One thread per target: the walk over all M markers, writing each marker's
-// slot masks (a0, a1 bits of the pairs' two haplotypes) at smasks[m][s] and,
-// when pairs is given, the pairs at pairs[s][m][L][2].
-__global__ void target_select_kernel(const uint8_t* __restrict__ geno, uint32_t B, uint32_t M, uint32_t N,
-                                     uint32_t W, uint32_t L, const uint32_t* __restrict__ prefix,
-                                     const uint32_t* __restrict__ panel, const uint32_t* __restrict__ rank_bits,
-                                     const uint32_t* __restrict__ rank_zeros, SlotMasks* __restrict__ smasks,
-                                     uint32_t* __restrict__ pairs) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= B) return;
-    const uint8_t* g = geno + (uint64_t)s * M;
+// The walk: one lane per target over all M markers, its position p in the order
+// of every marker written at smasks[m][s].pad for target_slots_kernel.
+// Bound: a chain of two dependent reads a marker (the word and the zero count at
+// p). kStage: the rank rows of a block of markers and the targets' codes are staged
+// in shared memory for the CTA's 32 targets, by warps that do nothing else, a block
+// ahead, so the chain waits for shared memory and not for L2. Rows of more than kWalkWords words are
+// read where they lie: 32 targets use a small part of such a row.
+// 512 targets x 4,003 markers, 1,024 haplotypes: 0.54 ms and 0.03 for the slots,
+// 5.2 when one thread a target read its ranks and its slots from L2 in one loop.
+// Not kept: rows fetched and codes loaded by the walking warp (1.57 ms), two blocks
+// of eight markers waited for whole (0.84), codes in the walking warp's registers
+// (0.62: its outstanding loads share a counter, so it waits for the youngest).
+constexpr uint32_t kWalkBlock = 4;    // markers per staged block
+constexpr uint32_t kWalkRing = 4;     // blocks in shared memory: one walked, three on their way
+constexpr uint32_t kWalkWords = 340;  // the blocks' rows and the codes stay under 48 KB
+constexpr uint32_t kWalkPrep = 3;     // staging warps
+constexpr uint32_t kWalkChunk = 8;    // blocks of codes staged at a time: 32 markers
+constexpr uint32_t kCodeRow = 36;     // bytes of a target's staged codes: an odd number of words, no bank conflicts
+
+template <bool kStage>
+__global__ void __launch_bounds__(kStage ? 32 * (1 + kWalkPrep) : 32)
+    target_walk_kernel(const uint8_t* __restrict__ geno, uint32_t B, uint32_t M, uint32_t N, uint32_t W,
+                       const uint32_t* __restrict__ rank_bits, const uint32_t* __restrict__ rank_zeros,
+                       SlotMasks* __restrict__ smasks) {
+    extern __shared__ __align__(16) uint32_t rows[];  // [kWalkRing]{[kWalkBlock][W] bits, [kWalkBlock][W + 1] zero counts}
+    __shared__ uint8_t codes[kStage ? 2 : 1][32 * kCodeRow];  // by chunk parity
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t part = kWalkBlock * (2 * W + 1);
+    const uint32_t NB = (M + kWalkBlock - 1) / kWalkBlock;
+    if (kStage && threadIdx.x >= 32) {
+        const uint32_t t = threadIdx.x - 32;
+        // a block's rows lie one after the other, from a 16-byte boundary (W is a multiple of 4)
+        auto fetch = [&](uint32_t b) {
+            if (b < NB) {
+                const uint32_t m0 = b * kWalkBlock, n = min(kWalkBlock, M - m0);
+                uint32_t* to = rows + b % kWalkRing * part;
+                const uint32_t* fb = rank_bits + (uint64_t)m0 * W;
+                const uint32_t* fz = rank_zeros + (uint64_t)m0 * (W + 1);
+                for (uint32_t i = 4 * t; i < n * W; i += 4 * 32 * kWalkPrep)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + i)),
+                                 "l"(fb + i) : "memory");
+                to += kWalkBlock * W;
+                const uint32_t whole = n * (W + 1) & ~3u;
+                for (uint32_t i = 4 * t; i < whole; i += 4 * 32 * kWalkPrep)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + i)),
+                                 "l"(fz + i) : "memory");
+                if (whole + t < n * (W + 1)) to[whole + t] = fz[whole + t];
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        // codes: rows of 32 markers, a warp a row; a chunk's loads are issued when the one before it is
+        // first walked and put into shared memory when that one is last walked
+        constexpr uint32_t kRows = (32 + kWalkPrep - 1) / kWalkPrep;
+        uint8_t got[kRows];
+        auto load = [&](uint32_t chunk) {
+            const uint32_t m = chunk * 32 + lane;
+#pragma unroll
+            for (uint32_t i = 0; i < kRows; ++i) {
+                const uint32_t r = t / 32 + i * kWalkPrep, s = blockIdx.x * 32 + r;
+                got[i] = r < 32 && s < B && m < M ? geno[(uint64_t)s * M + m] : 3;
+            }
+        };
+        auto put = [&](uint32_t chunk) {
+#pragma unroll
+            for (uint32_t i = 0; i < kRows; ++i) {
+                const uint32_t r = t / 32 + i * kWalkPrep;
+                if (r < 32) codes[chunk & 1u][r * kCodeRow + lane] = got[i];
+            }
+        };
+        for (uint32_t b = 0; b + 1 < kWalkRing; ++b) fetch(b);
+        load(0);
+        put(0);
+        for (uint32_t b = 0; b < NB; ++b) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kWalkRing - 2) : "memory");
+            __syncthreads();  // block b is there; block b - 1 has been walked
+            fetch(b + kWalkRing - 1);
+            if (b % kWalkChunk == 0) load(b / kWalkChunk + 1);
+            if (b % kWalkChunk == kWalkChunk - 1) put(b / kWalkChunk + 1);
+        }
+        return;
+    }
+    const uint32_t s = blockIdx.x * 32 + lane;
+    const bool live = s < B;
+    const uint8_t* g = geno + (uint64_t)(live ? s : B - 1) * M;
+    SlotMasks* out = smasks + (live ? s : B - 1);  // a lane past the batch's end repeats its last target
     uint32_t p = 0;
-    for (uint32_t m = 0; m < M; ++m) {
-        const uint32_t* bits = rank_bits + (uint64_t)m * W;
-        const uint32_t* zeros = rank_zeros + (uint64_t)m * (W + 1);
-        const uint32_t Z = zeros[W];
-        const uint32_t zb = p < N ? zeros[p >> 5] + __popc(~bits[p >> 5] & ((1u << (p & 31)) - 1u)) : Z;
-        const uint32_t q = p < N ? p : N - 1;
-        const uint32_t code = g[m];
-        const uint32_t xt = code == 0 ? 0u : code == 2 ? 1u : ((bits[q >> 5] >> (q & 31)) & 1u);
-        p = xt ? Z + (p - zb) : zb;
-        const uint32_t* row = prefix + (uint64_t)m * N;
-        const uint32_t* prow = panel + (uint64_t)m * W;
-        uint32_t s0 = 0;
-        if (L <= N) s0 = min(p > L / 2 ? p - L / 2 : 0u, N - L);
-        uint32_t a0 = 0, a1 = 0;
-        for (uint32_t r = 0; r < L; ++r) {
-            const uint32_t h0 = L <= N ? row[s0 + r] : row[r % N];
-            const uint32_t h1 = (h0 + 1) % N;
-            a0 |= ((prow[h0 >> 5] >> (h0 & 31)) & 1u) << r;
-            a1 |= ((prow[h1 >> 5] >> (h1 & 31)) & 1u) << r;
-            if (pairs) {
-                uint32_t* o = pairs + (((uint64_t)s * M + m) * L + r) * 2;
-                o[0] = h0;
-                o[1] = h1;
+    for (uint32_t b = 0; b < NB; ++b) {
+        if (kStage) __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < kWalkBlock; ++j) {
+            const uint32_t m = b * kWalkBlock + j;
+            if (m < M) {
+                const uint32_t* bits = kStage ? rows + b % kWalkRing * part + j * W : rank_bits + (uint64_t)m * W;
+                const uint32_t* zeros = kStage ? rows + b % kWalkRing * part + kWalkBlock * W + j * (W + 1)
+                                               : rank_zeros + (uint64_t)m * (W + 1);
+                const uint32_t Z = zeros[W];
+                const uint32_t c = kStage ? codes[(b / kWalkChunk) & 1u][lane * kCodeRow + (b % kWalkChunk) * kWalkBlock + j] : g[m];
+                const uint32_t q = min(p, N - 1);
+                const uint32_t word = bits[q >> 5];
+                const uint32_t zb = p < N ? zeros[q >> 5] + __popc(~word & ((1u << (p & 31)) - 1u)) : Z;
+                const uint32_t xt = c == 0 ? 0u : c == 2 ? 1u : ((word >> (q & 31)) & 1u);
+                p = xt ? Z + (p - zb) : zb;
+                out->pad = p;
+                out += B;
             }
         }
-        smasks[(uint64_t)m * B + s] = SlotMasks{a0, a1, 0u, 0u};
     }
+}
+
+// The slots at every (marker, target) position of the walk, one thread each,
+// targets fastest: the masks (a0, a1 bits of the pairs' two haplotypes) at
+// smasks[m][s] and, when pairs is given, the pairs at pairs[s][m][L][2].
+__global__ void __launch_bounds__(256) target_slots_kernel(uint32_t B, uint32_t M, uint32_t N, uint32_t W, uint32_t L,
+                                                           const uint32_t* __restrict__ prefix,
+                                                           const uint32_t* __restrict__ panel,
+                                                           SlotMasks* __restrict__ smasks, uint32_t* __restrict__ pairs) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (uint64_t)M * B) return;
+    const uint32_t m = (uint32_t)(i / B), s = (uint32_t)(i % B);
+    const uint32_t p = smasks[i].pad;
+    const uint32_t* row = prefix + (uint64_t)m * N;
+    const uint32_t* prow = panel + (uint64_t)m * W;
+    uint32_t s0 = 0;
+    if (L <= N) s0 = min(p > L / 2 ? p - L / 2 : 0u, N - L);
+    uint32_t a0 = 0, a1 = 0;
+    for (uint32_t r = 0; r < L; ++r) {
+        const uint32_t h0 = L <= N ? row[s0 + r] : row[r % N];
+        const uint32_t h1 = (h0 + 1) % N;
+        a0 |= ((prow[h0 >> 5] >> (h0 & 31)) & 1u) << r;
+        a1 |= ((prow[h1 >> 5] >> (h1 & 31)) & 1u) << r;
+        if (pairs) {
+            uint32_t* o = pairs + (((uint64_t)s * M + m) * L + r) * 2;
+            o[0] = h0;
+            o[1] = h1;
+        }
+    }
+    smasks[i] = SlotMasks{a0, a1, 0u, 0u};
 }
 
 }  // namespace
@@ -226,8 +324,16 @@ cudaError_t launch_target_select(const uint8_t* d_geno, uint32_t B, uint32_t M, 
                                  const uint32_t* d_prefix, const uint32_t* d_panel, const uint32_t* d_bits,
                                  const uint32_t* d_zeros, SlotMasks* d_smasks, uint32_t* d_pairs, cudaStream_t s) {
     if (B == 0) return cudaSuccess;
-    target_select_kernel<<<(B + 127) / 128, 128, 0, s>>>(d_geno, B, M, N, W, L, d_prefix, d_panel, d_bits, d_zeros,
-                                                        d_smasks, d_pairs);
+    if (W <= kWalkWords)
+        target_walk_kernel<true><<<(B + 31) / 32, 32 * (1 + kWalkPrep), kWalkRing * kWalkBlock * (2 * W + 1) * 4, s>>>(
+            d_geno, B, M, N, W, d_bits, d_zeros, d_smasks);
+    else
+        target_walk_kernel<false><<<(B + 31) / 32, 32, 0, s>>>(d_geno, B, M, N, W, d_bits, d_zeros, d_smasks);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const uint64_t grid = ((uint64_t)M * B + 255) / 256;
+    if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
+    target_slots_kernel<<<(uint32_t)grid, 256, 0, s>>>(B, M, N, W, L, d_prefix, d_panel, d_smasks, d_pairs);
     return cudaGetLastError();
 }
 

@@ -142,3 +142,20 @@ def test_full_chain_segments(engine, L, M, B, C, per_gap):
         one_pass = tight.impute(codes, p, hap_prob=True)
     for key in got:
         assert np.array_equal(got[key], one_pass[key]), key
+
+
+# per-target slots: rows staged in shared memory (up to 10,880 haplotypes) and read where they lie, lengths
+# around the staged blocks (4) and code chunks (32), targets around a warp
+@pytest.mark.parametrize("N_,M,B,L", [(2, 5, 3, 4), (33, 1, 1, 2), (300, 7, 31, 8), (300, 8, 32, 8), (300, 9, 33, 32),
+                                      (1024, 65, 40, 16), (10880, 20, 5, 8), (10881, 20, 34, 8)])
+def test_target_walk(engine, N_, M, B, L):
+    panel, pos, _ = synth.make_panel(M, N_, 8, seed=M + N_)
+    rng = np.random.default_rng(N_)
+    codes = rng.integers(0, 5, (B, M)).astype(np.uint8)
+    engine.upload_panel(panel)
+    engine.set_map(pos)
+    engine.pbwt_build(store_index=True)
+    got = engine.select_states_target(L, codes)
+    prefix = engine.prefix_rows()
+    for b in range(B):
+        assert np.array_equal(got[b], oracle.select_pairs_target(prefix, panel, codes[b], L)), b
