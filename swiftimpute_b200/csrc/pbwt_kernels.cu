@@ -72,7 +72,8 @@ constexpr int kSweepThreads = 1024;
 template <bool kSmemPerm, int kE>
 __global__ void __launch_bounds__(kSweepThreads, 1)
 pbwt_sweep_kernel(const uint32_t* __restrict__ panel_all, const SweepJob* __restrict__ jobs, uint32_t N, uint32_t W,
-                  uint32_t E, const uint32_t* __restrict__ init, uint32_t* __restrict__ head_all,
+                  uint32_t E, const uint32_t* __restrict__ init, const uint16_t* __restrict__ init16,
+                  uint32_t* __restrict__ head_all,
                   uint32_t* __restrict__ prefix, unsigned long long* __restrict__ row_hash,
                   uint32_t* __restrict__ gperm_all) {
     extern __shared__ __align__(16) uint32_t smem[];
@@ -93,8 +94,9 @@ pbwt_sweep_kernel(const uint32_t* __restrict__ panel_all, const SweepJob* __rest
 
     if (job.init_off == kIota) {
         for (uint32_t i = t; i < N; i += blockDim.x) cur[i] = i;  // iota, pbwt_index.cpp:226
-    } else {
-        for (uint32_t i = t; i < N; i += blockDim.x) cur[i] = init[job.init_off + i];  // a later segment's start
+    } else {  // a later segment's start
+        for (uint32_t i = t; i < N; i += blockDim.x)
+            cur[i] = init16 ? init16[job.init_off + i] : init[job.init_off + i];
     }
     for (uint32_t i = t; i < W; i += blockDim.x) rows[i] = panel[i];
     __syncthreads();
@@ -211,16 +213,200 @@ pbwt_sweep_kernel(const uint32_t* __restrict__ panel_all, const SweepJob* __rest
 // alleles over [a, b) read as a key (marker b-1 most significant): the order
 // swept from 0 .. N-1 over the segment alone ranks those keys, and the order
 // before a breaks their ties. So the build runs in three passes:
-//   groups   every segment but the last, on its own CTA: the sweep from
-//            0 .. N-1 over its markers, carrying for each entry the index of
-//            its group (haplotypes equal over the markers swept so far); the
-//            final group index of each haplotype is the key rank above;
-//   compose  for each segment in turn, one CTA: the order before the next
-//            segment = this segment's start order stably sorted by group index
-//            (an LSD radix sort, 8-bit digits);
+//   ranks    every segment but the last, on its own CTA: the haplotypes sorted
+//            from 0 .. N-1 by their keys, and the rank of each one's key among
+//            the segment's different keys;
+//   compose  the orders before the segments. Ranks over several segments compose
+//            like keys: the rank over segments i .. j is that of the pair (rank
+//            over k+1 .. j, rank over i .. k), so log2(segments) rounds of doubled
+//            reach give every segment's rank over all markers before its end, and
+//            with it the order before the next one;
 //   sweep    every segment on its own CTA from its start order, writing its
 //            rows (pbwt_sweep_kernel with init_off).
 // The result is bit-identical to one sweep over all markers.
+// Panels whose sort state does not fit a CTA's shared memory (about 20,000
+// haplotypes) take pbwt_group_kernel for the ranks (a sweep that carries the
+// groups of equal keys) and pbwt_compose_kernel, one segment after the other.
+
+constexpr uint32_t kSortThreads = 1024;
+constexpr uint32_t kSortWarps = kSortThreads / 32;
+constexpr uint32_t kCntRow = kSortWarps + 1;  // counter row stride: a warp's counters of different digits in different banks
+constexpr size_t kSortFixed = (size_t)256 * kCntRow * 4 + 32 * 4;
+
+// One stable counting-sort pass of src by an 8-bit digit of each element into
+// dst, by all threads. Warp w owns the contiguous elements [w c, w c + c), so
+// ranks within a digit follow the input order: per-warp digit counts, their scan
+// in (digit, warp) order, then each warp places its elements 32 at a time, lanes
+// with equal digits ranked by lane (match_any).
+template <class Digit>
+__device__ __forceinline__ void sort_pass(const uint16_t* src, uint16_t* dst, uint32_t N, uint32_t* cnt, uint32_t* wsum,
+                                          Digit digit) {
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t c = (N + kSortWarps - 1) / kSortWarps;
+    const uint32_t e0 = min(N, warp * c), e1 = min(N, e0 + c);
+    for (uint32_t i = t; i < 256 * kCntRow; i += kSortThreads) cnt[i] = 0u;
+    __syncthreads();
+    for (uint32_t i = e0 + lane; i < e1; i += 32) atomicAdd(&cnt[digit(src[i]) * kCntRow + warp], 1u);
+    __syncthreads();
+    // exclusive scan of the 8,192 counts in (digit, warp) order, 8 per thread
+    uint32_t* mine = cnt + (t >> 2) * kCntRow + (t & 3u) * 8;
+    uint32_t loc[8], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { loc[j] = mine[j]; sum += loc[j]; }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    const uint32_t wt = wsum[lane];
+    uint32_t wi = wt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, wi, o);
+        if (lane >= (uint32_t)o) wi += y;
+    }
+    uint32_t run = __shfl_sync(0xffffffffu, wi - wt, warp) + incl - sum;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { mine[j] = run; run += loc[j]; }
+    __syncthreads();
+    for (uint32_t b0 = e0; b0 < e1; b0 += 32) {  // warp-private counters
+        const uint32_t i = b0 + lane;
+        const bool ok = i < e1;
+        const uint16_t v = ok ? src[i] : (uint16_t)0;
+        const uint32_t d = ok ? digit(v) : 256u + lane;  // idle lanes match nobody
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        uint32_t base = 0;
+        if (ok) base = cnt[d * kCntRow + warp];
+        if (ok) dst[base + __popc(peers & ((1u << lane) - 1u))] = v;
+        __syncwarp();
+        if (ok && (peers >> lane) == 1u) cnt[d * kCntRow + warp] = base + __popc(peers);  // the highest lane of the group
+        __syncwarp();
+    }
+    __syncthreads();
+}
+
+// rank[ord[i]] = number of i' <= i (i' > 0) where differs(ord[i' - 1], ord[i']),
+// by all threads; differs may read rank, which changes only after every thread
+// has read it.
+template <class Differs>
+__device__ __forceinline__ void dense_ranks(const uint16_t* ord, uint16_t* rank, uint32_t N, uint32_t* wsum, Differs differs) {
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t E = (N + kSortThreads - 1) / kSortThreads;
+    const uint32_t i0 = min(N, t * E), i1 = min(N, i0 + E);
+    uint32_t n = 0, bits = 0;  // E <= 24 at the sizes that fit shared memory
+    for (uint32_t i = i0; i < i1; ++i)
+        if (i && differs(ord[i - 1], ord[i])) {
+            ++n;
+            bits |= 1u << (i - i0);
+        }
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    const uint32_t wt = wsum[lane];
+    uint32_t wi = wt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, wi, o);
+        if (lane >= (uint32_t)o) wi += y;
+    }
+    uint32_t r = __shfl_sync(0xffffffffu, wi - wt, warp) + incl - n;
+    for (uint32_t i = i0; i < i1; ++i) {
+        r += (bits >> (i - i0)) & 1u;
+        rank[ord[i]] = (uint16_t)r;
+    }
+    __syncthreads();
+}
+
+// Ranks pass: jobs[b] = {m0, len, -, -}. An LSD radix sort over the segment's
+// markers, eight a pass (a haplotype's byte is its alleles at those markers, the
+// last one most significant), with the ranks of the keys so far carried along.
+// Bound by latency: about ten block barriers a pass of eight markers. 4,432
+// haplotypes x 50,000 markers in 148 segments: 0.35 ms (a sweep that carried
+// groups of equal keys, marker by marker, took 1.42), the composition's eight
+// rounds 0.15 (147 sorts one after the other: 4.43), the sweep 0.63. With 296
+// segments, two CTAs an SM: 0.32 + 0.26 + 0.61; with the next rows fetched a pass
+// ahead: 0.37 for the ranks.
+__global__ void __launch_bounds__(kSortThreads, 1)
+pbwt_rank_kernel(const uint32_t* __restrict__ panel_all, const SweepJob* __restrict__ jobs, uint32_t N, uint32_t W,
+                 uint16_t* __restrict__ order_all, uint16_t* __restrict__ rank_all) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    uint32_t* rows = smem;                                    // [8][W]
+    uint32_t* cnt = rows + 8 * W;                             // [256][kCntRow]
+    uint32_t* wsum = cnt + 256 * kCntRow;                     // [32]
+    uint16_t* cur = reinterpret_cast<uint16_t*>(wsum + 32);   // haplotype at each position
+    uint16_t* nxt = cur + N;
+    uint16_t* rank = nxt + N;                                 // by haplotype
+    uint8_t* dig = reinterpret_cast<uint8_t*>(rank + N);      // by haplotype
+    const SweepJob job = jobs[blockIdx.x];
+    const uint32_t* panel = panel_all + (uint64_t)job.m0 * W;
+    const uint32_t t = threadIdx.x;
+    for (uint32_t i = t; i < N; i += kSortThreads) { cur[i] = (uint16_t)i; rank[i] = 0; }
+    for (uint32_t b = 0; b < job.len; b += 8) {
+        const uint32_t nr = min(8u, job.len - b);
+        const uint4* from = reinterpret_cast<const uint4*>(panel + (uint64_t)b * W);  // rows follow each other, 16-byte aligned
+        for (uint32_t i = t; i < nr * W / 4; i += kSortThreads) reinterpret_cast<uint4*>(rows)[i] = __ldg(from + i);
+        __syncthreads();
+        for (uint32_t h = t; h < N; h += kSortThreads) {
+            uint32_t x = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i)
+                if (i < nr) x |= ((rows[i * W + (h >> 5)] >> (h & 31)) & 1u) << i;
+            dig[h] = (uint8_t)x;
+        }
+        __syncthreads();
+        sort_pass(cur, nxt, N, cnt, wsum, [&](uint32_t h) { return (uint32_t)dig[h]; });
+        dense_ranks(nxt, rank, N, wsum, [&](uint32_t x, uint32_t y) { return dig[x] != dig[y] || rank[x] != rank[y]; });
+        uint16_t* z = cur; cur = nxt; nxt = z;
+    }
+    for (uint32_t i = t; i < N; i += kSortThreads) {
+        order_all[(uint64_t)blockIdx.x * N + i] = cur[i];
+        rank_all[(uint64_t)blockIdx.x * N + i] = rank[i];
+    }
+}
+
+// One round of the composition: block j's order and ranks over the d segments
+// ending at j become those over the 2 d segments ending at j (or over all of
+// them): the order over the d segments ending at j - d, stably sorted by j's rank,
+// ranked by the pair. Blocks below d cover all of theirs already.
+__global__ void __launch_bounds__(kSortThreads, 1)
+pbwt_double_kernel(const uint16_t* __restrict__ order_in, const uint16_t* __restrict__ rank_in, uint32_t N, uint32_t d,
+                   uint32_t bits, uint16_t* __restrict__ order_out, uint16_t* __restrict__ rank_out) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    const uint32_t j = blockIdx.x, t = threadIdx.x;
+    const uint16_t* rj = rank_in + (uint64_t)j * N;
+    uint16_t* oo = order_out + (uint64_t)j * N;
+    uint16_t* ro = rank_out + (uint64_t)j * N;
+    if (j < d) {
+        const uint16_t* oj = order_in + (uint64_t)j * N;
+        for (uint32_t i = t; i < N; i += kSortThreads) { oo[i] = oj[i]; ro[i] = rj[i]; }
+        return;
+    }
+    uint32_t* cnt = smem;
+    uint32_t* wsum = cnt + 256 * kCntRow;
+    uint16_t* cur = reinterpret_cast<uint16_t*>(wsum + 32);
+    uint16_t* nxt = cur + N;
+    uint16_t* hi = nxt + N;  // by haplotype
+    uint16_t* lo = hi + N;
+    const uint16_t* ol = order_in + (uint64_t)(j - d) * N;
+    const uint16_t* rl = rank_in + (uint64_t)(j - d) * N;
+    for (uint32_t i = t; i < N; i += kSortThreads) { cur[i] = ol[i]; hi[i] = rj[i]; lo[i] = rl[i]; }
+    __syncthreads();
+    for (uint32_t sh = 0; sh < bits; sh += 8) {
+        sort_pass(cur, nxt, N, cnt, wsum, [&](uint32_t h) { return ((uint32_t)hi[h] >> sh) & 255u; });
+        uint16_t* z = cur; cur = nxt; nxt = z;
+    }
+    // nxt takes the ranks, by haplotype
+    dense_ranks(cur, nxt, N, wsum, [&](uint32_t x, uint32_t y) { return hi[x] != hi[y] || lo[x] != lo[y]; });
+    for (uint32_t i = t; i < N; i += kSortThreads) { oo[i] = cur[i]; ro[i] = nxt[i]; }
+}
 
 // Block-wide exclusive scans of per-thread values over kSweepThreads threads:
 // a warp scan, one barrier, and every warp scanning the warp totals itself.
@@ -264,8 +450,9 @@ __device__ __forceinline__ void block_scan(uint32_t (&v)[K], const bool (&is_max
     }
 }
 
-// Groups pass: jobs[b] = {m0, len, -, -} swept from 0 .. N-1 with group
-// indices; gid_all[b][h] = the index of haplotype h's group at the end.
+// Ranks pass of large panels: jobs[b] = {m0, len, -, -} swept from 0 .. N-1 with
+// the indices of the groups of equal keys; gid_all[b][h] = the index of haplotype
+// h's group at the end.
 // Entries live in shared memory when 4 N words fit, else in scratch [b][4][N].
 template <bool kSmem>
 __global__ void __launch_bounds__(kSweepThreads, 1)
@@ -350,7 +537,7 @@ pbwt_group_kernel(const uint32_t* __restrict__ panel_all, const SweepJob* __rest
     for (uint32_t i = t; i < N; i += blockDim.x) gid[cur[i]] = cg[i];
 }
 
-// Compose: next = order stably sorted by gid[order[r]]; one CTA of 1024
+// Composition of large panels: next = order stably sorted by gid[order[r]]; one CTA of 1024
 // threads, LSD radix sort with 8-bit digits over the bits of N - 1. Warp w
 // owns the contiguous elements [w c, w c + c) of every pass, so ranks within a
 // digit follow the input order: per-warp digit counts, their scan in (digit,
@@ -465,8 +652,8 @@ size_t pbwt_sweep_smem_bytes(uint32_t N, uint32_t W) {
 // One CTA per job (device array d_jobs[n_jobs]); head must be zero-filled for
 // rows shorter than kHead; d_perm_scratch holds 2 N words per job.
 cudaError_t launch_pbwt_sweep(const uint32_t* d_panel, const SweepJob* d_jobs, uint32_t n_jobs, uint32_t N,
-                              uint32_t W, const uint32_t* d_init, uint32_t* d_head, uint32_t* d_prefix,
-                              unsigned long long* d_hash, uint32_t* d_perm_scratch, cudaStream_t s) {
+                              uint32_t W, const uint32_t* d_init, const uint16_t* d_init16, uint32_t* d_head,
+                              uint32_t* d_prefix, unsigned long long* d_hash, uint32_t* d_perm_scratch, cudaStream_t s) {
     uint32_t T = ((N + 4 * 32 - 1) / (4 * 32)) * 32;  // ~4 entries per thread, 128..1024 threads
     T = T < 128 ? 128 : (T > kSweepThreads ? kSweepThreads : T);
     const uint32_t E = (N + T - 1) / T;
@@ -477,7 +664,7 @@ cudaError_t launch_pbwt_sweep(const uint32_t* d_panel, const SweepJob* d_jobs, u
     auto go = [&](auto kernel, size_t smem, uint32_t* gp) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kernel<<<n_jobs, T, smem, s>>>(d_panel, d_jobs, N, W, E, d_init, d_head, d_prefix, d_hash, gp);
+        kernel<<<n_jobs, T, smem, s>>>(d_panel, d_jobs, N, W, E, d_init, d_init16, d_head, d_prefix, d_hash, gp);
         return cudaSuccess;
     };
     cudaError_t e;
@@ -492,6 +679,32 @@ cudaError_t launch_pbwt_sweep(const uint32_t* d_panel, const SweepJob* d_jobs, u
                     : go(pbwt_sweep_kernel<false, 0>, small, d_perm_scratch);
     }
     if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+// Shared memory of the sorted build's CTAs (the larger of the two kernels').
+size_t pbwt_sort_smem_bytes(uint32_t N, uint32_t W) {
+    const size_t ranks = (size_t)8 * W * 4 + kSortFixed + (size_t)7 * N + 16, pairs = kSortFixed + (size_t)8 * N + 16;
+    return ranks > pairs ? ranks : pairs;
+}
+
+// Orders before segments 1 .. n_jobs of a panel whose sort state fits shared
+// memory: d_buf holds 4 n_jobs N 16-bit words; *d_orders [n_jobs][N] points into it.
+cudaError_t launch_pbwt_orders(const uint32_t* d_panel, const SweepJob* d_jobs, uint32_t n_jobs, uint32_t N, uint32_t W,
+                               uint16_t* d_buf, const uint16_t** d_orders, cudaStream_t s) {
+    const size_t sm = pbwt_sort_smem_bytes(N, W), words = (size_t)n_jobs * N;
+    uint16_t *o = d_buf, *r = o + words, *o2 = r + words, *r2 = o2 + words;
+    cudaError_t e = cudaFuncSetAttribute(pbwt_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(pbwt_double_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    pbwt_rank_kernel<<<n_jobs, kSortThreads, sm, s>>>(d_panel, d_jobs, N, W, o, r);
+    const uint32_t bits = N > 1 ? 32u - (uint32_t)__builtin_clz(N - 1) : 0u;  // ranks are < N
+    for (uint32_t d = 1; d < n_jobs; d *= 2) {
+        pbwt_double_kernel<<<n_jobs, kSortThreads, sm, s>>>(o, r, N, d, bits, o2, r2);
+        uint16_t* z = o; o = o2; o2 = z;
+        z = r; r = r2; r2 = z;
+    }
+    *d_orders = o;
     return cudaGetLastError();
 }
 

@@ -165,13 +165,18 @@ bool region_first_gap_ok(const si_ctx* ctx, const si_impute_params* p, uint32_t 
 // Kernel launchers (pbwt_kernels.cu, select_kernels.cu, fb_kernels.cu).
 cudaError_t launch_pack_panel(const uint8_t* d_u8, uint32_t M, uint32_t N, uint32_t W, uint32_t* d_words,
                               cudaStream_t s);
-// d_init: the orders jobs with init_off != kIota start from (may be null when none does)
+// d_init or d_init16: the orders jobs with init_off != kIota start from (both null when none does)
 cudaError_t launch_pbwt_sweep(const uint32_t* d_panel, const SweepJob* d_jobs, uint32_t n_jobs, uint32_t N,
-                              uint32_t W, const uint32_t* d_init, uint32_t* d_head, uint32_t* d_prefix,
+                              uint32_t W, const uint32_t* d_init, const uint16_t* d_init16, uint32_t* d_head,
+                              uint32_t* d_prefix,
                               unsigned long long* d_hash, uint32_t* d_perm_scratch, cudaStream_t s);
 size_t pbwt_sweep_smem_bytes(uint32_t N, uint32_t W);
 size_t pbwt_group_smem_bytes(uint32_t N, uint32_t W);
-// Segmented whole-panel sweep (pbwt_kernels.cu): per segment the groups of
+size_t pbwt_sort_smem_bytes(uint32_t N, uint32_t W);
+cudaError_t launch_pbwt_orders(const uint32_t* d_panel, const SweepJob* d_jobs, uint32_t n_jobs, uint32_t N, uint32_t W,
+                               uint16_t* d_buf, const uint16_t** d_orders, cudaStream_t s);
+// Segmented whole-panel sweep (pbwt_kernels.cu): the segments' start orders where
+// a CTA's shared memory holds the sort state; else, per segment, the groups of
 // haplotypes equal over its markers, swept from 0 .. N-1 (d_gid [n_jobs][N],
 // by haplotype; d_scratch 4 N words per job), and the composition of an order
 // with one segment's groups (a stable sort by group; d_sortbuf 4 N words).

@@ -159,3 +159,21 @@ def test_target_walk(engine, N_, M, B, L):
     prefix = engine.prefix_rows()
     for b in range(B):
         assert np.array_equal(got[b], oracle.select_pairs_target(prefix, panel, codes[b], L)), b
+
+
+# the index built from sorted segments (up to about 20,000 haplotypes) and from swept groups: segment counts
+# around powers of two, a last segment of any length, passes of eight markers with a remainder, many equal
+# haplotypes (long groups) and none
+@pytest.mark.parametrize("M,N_", [(127, 100), (128, 100), (129, 33), (192, 2), (256, 1025), (257, 5), (320, 64),
+                                  (1000, 1024), (9600, 300), (9472, 31), (200, 20000), (140, 27000)])
+@pytest.mark.parametrize("p1", [0.02, 0.5])
+def test_index_segments(engine, M, N_, p1):
+    rng = np.random.default_rng(M + N_)
+    panel = (rng.random((M, N_)) < p1).astype(np.uint8)
+    panel[:, N_ // 2:] = panel[:, :N_ - N_ // 2]  # every haplotype twice: ties keep their order
+    engine.upload_panel(panel)
+    engine.pbwt_build(store_index=N_ <= 1025, row_hashes=True)
+    rows, hashes = oracle.pbwt_build_packed(synth.pack_panel(panel), N_)[:2]
+    assert np.array_equal(engine.row_hashes(), hashes)
+    if N_ <= 1025:
+        assert np.array_equal(engine.prefix_rows(), oracle.pbwt_build(panel))
