@@ -830,7 +830,11 @@ __global__ void __launch_bounds__(kChainThreads, LM <= 16 ? 5 : 3) anchor_chain_
 // -> now: 10,000 x 50,000 (L = 8) 4.06 -> 2.35 ms (writing its 3 GB would take
 // 0.47); 2,003 x 30,011 0.76 -> 0.41; 4,000 x 20,000 (L = 16) 1.27 -> 0.68; 1,500
 // x 6,007 (L = 32, alleles only) 0.22 -> 0.18; one target x 1,644 98 -> 57 us;
-// 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 1.12 ms.
+// 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 0.55 ms.
+
+// Lanes that take an anchor together, each lane by itself: 131 x 7,919 with sites of their own takes
+// 1.12 ms when a lane takes its anchors alone, 0.79 with 4, 0.83 with 8, 1.00 with 16.
+constexpr int kTurn = 4;
 
 // high word of farg' for a uniform run and for a negligible floor
 constexpr uint32_t kInfHi = 0x7ff00000u;
@@ -1089,14 +1093,16 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     st.P = reinterpret_cast<uint32_t*>(st.U + 32);
     st.E = st.P + (C + 1) * 32;
 
-    const uint32_t SG = (A.B + 31) / 32, SC = (SG + nw - 1) / nw;  // sample groups, CTAs of one window group
+    // a warp takes A.rows samples (a divisor of 32): SW warps and SC CTAs of one window group
+    const uint32_t SW = (A.B + A.rows - 1) / A.rows, SC = (SW + nw - 1) / nw;
     const unsigned long long grp = blockIdx.x / SC;
-    const uint32_t g0 = blockIdx.x % SC * nw, g = g0 + warp;
-    const uint32_t cta_threads = 32 * min(nw, SG - g0);  // the warps with samples
-    if (g >= SG) return;  // whole warp
-    // a lane past the batch's end repeats its last sample, and writes nothing
-    const bool real = g * 32 + lane < A.B;
-    const uint32_t s = real ? g * 32 + lane : A.B - 1;
+    const uint32_t w0cta = blockIdx.x % SC * nw;
+    const uint32_t cta_threads = 32 * min(nw, SW - w0cta);  // the warps with samples
+    if (w0cta + warp >= SW) return;  // whole warp
+    const uint32_t row0 = (w0cta + warp) * A.rows, g = row0 / 32;
+    // a lane past the warp's samples or the batch's end repeats one of them, and writes nothing
+    const bool real = lane < A.rows && row0 + lane < A.B;
+    const uint32_t s = min(row0 + (lane & (A.rows - 1)), A.B - 1);
     bool live = grp * K < A.max_windows;
     View v{};
     if (!kPlain) v = view_of(A, s);
@@ -1402,7 +1408,7 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
         auto warp_value = [&](uint32_t x) { return __reduce_max_sync(kAll, x); };
         uint32_t um = warp_value(m), u0 = um, u1 = warp_value(p1);
         const uint32_t uend = warp_value(mend);
-        const uint32_t rows = min(32u, A.B - g * 32);
+        const uint32_t rows = min(A.rows, A.B - row0);
         // the current run's floor on one form for every lane, so that a step needs no branch: -3e38
         // stands for a negligible floor (F = 0), 3e38 for a uniform run (X w' = 0 there, Y F + 1 = 1)
         auto one_form = [&] {
@@ -1583,7 +1589,7 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
                 const unsigned long long od = out + utb + lane;
 #pragma unroll 4
                 for (uint32_t r = 0; r < rows; ++r) {
-                    const unsigned long long rd = kPlain ? (unsigned long long)(g * 32 + r) * A.M + utb + lane
+                    const unsigned long long rd = kPlain ? (unsigned long long)(row0 + r) * A.M + utb + lane
                                                          : __shfl_sync(kAll, od, r) - r + lane;
                     if (col) {
                         if (w_dos) A.dosage[rd] = tD[r * 36 + lane];
@@ -1601,39 +1607,35 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
         return;
     }
 
+    // ---- every lane by itself: lanes reach their anchors at different cells, and an anchor costs about
+    // three steps of cells, so those at one wait until kTurn of them (or all that still have cells in the
+    // tile) are there and take it together.
     uint32_t tbase = m & ~31u;
     for (;;) {
         const bool on = live && m < mend;
         if (!__any_sync(kAll, on)) break;
-        uint32_t tlo = 32, thi = 0;
-        if (on) {
-            const uint32_t tend = min(tbase + 32, mend);
-            tlo = m - tbase;
-            while (m < tend) {
-                if (m == p1) {
+        const uint32_t tend = min(tbase + 32, mend), tlo = on ? m - tbase : 32u;
+        for (;;) {
+            const bool more = on && m < tend, turn = more && m == p1;
+            const uint32_t turns = __ballot_sync(kAll, turn), steps = __ballot_sync(kAll, more && !turn);
+            if (!(turns | steps)) break;
+            if (!steps || __popc(turns) >= kTurn) {
+                if (turn) {
                     anchor(tabQS(tb, p1 - p0));
                     p0 = p1;
                     p1 = fr.z;
                     in_tab = p1 - p0 < tb.NT;
                 }
-                // cells [m, e) of the run, two per step when they pair up
+            } else if (more && !turn) {  // the next cells of the run, two per step when they pair up
                 const uint32_t e = min(p1, tend);
+                const bool two = (m & 1u) == 0u && m + 1 < e;
                 float4 qa, qb;
                 coeffs(m, qa, qb);
-                while (m < e) {
-                    const bool two = (m & 1u) == 0u && m + 1 < e;
-                    const uint32_t mn = m + (two ? 2u : 1u);
-                    float4 na = qa, nb = qb;
-                    if (mn < e) coeffs(mn, na, nb);  // the next step's coefficients in flight
-                    cells(m, two, qa, qb, m - tbase);
-                    qa = na;
-                    qb = nb;
-                    m = mn;
-                }
+                cells(m, two, qa, qb, m - tbase);
+                m += two ? 2u : 1u;
             }
-            thi = m - tbase;
         }
-        flush(tbase, tlo, thi, on);
+        flush(tbase, tlo, on ? m - tbase : 0u, on);
         tbase += 32;
     }
 }
@@ -1656,7 +1658,12 @@ cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
         if (e != cudaSuccess) return e;
     }
     const unsigned long long groups = ((unsigned long long)a.max_windows + a.K - 1) / a.K;
-    const unsigned long long grid = groups * ((typed_groups(a.B) + T / 32 - 1) / (T / 32));
+    // A batch of few warps gives each fewer samples, while that leaves at most two warps a scheduler:
+    // lanes at their own sites wait for fewer others (131 x 7,919: 0.79 ms with 32 samples a warp, 0.58
+    // with 8, 0.55 with 4, 0.75 with 2), and lanes in step lose nothing (444 x 1,644: 64 us and 60).
+    f.rows = 32;
+    while (f.rows > 4 && groups * ((a.B + f.rows / 2 - 1) / (f.rows / 2)) <= 8u * 148u) f.rows /= 2;
+    const unsigned long long grid = groups * (((a.B + f.rows - 1) / f.rows + T / 32 - 1) / (T / 32));
     if (grid == 0) return cudaSuccess;
     if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
     anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos><<<(uint32_t)grid, T, sm, s>>>(f);
