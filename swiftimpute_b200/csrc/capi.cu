@@ -20,19 +20,36 @@ si_status cuda_fail(si_ctx* ctx, cudaError_t e, const char* what) {
     return fail(ctx, e == cudaErrorMemoryAllocation ? SI_ERR_OUT_OF_MEMORY : SI_ERR_CUDA, m);
 }
 
+uint64_t reclaimable_bytes(const si_ctx* ctx) {
+    uint64_t b = ctx->bckpt.bytes + ctx->build.bytes;
+    for (auto& kv : ctx->sel)
+        if (kv.second.stale) b += kv.second.pairs.bytes + kv.second.masks.bytes + kv.second.g2.bytes + kv.second.raw.bytes;
+    return b;
+}
+
+void reclaim(si_ctx* ctx) {  // cudaFree waits for the kernels that use a buffer
+    dev_free(ctx, ctx->bckpt);
+    dev_free(ctx, ctx->build);
+    for (auto it = ctx->sel.begin(); it != ctx->sel.end();) {
+        if (!it->second.stale) { ++it; continue; }
+        for (DeviceBuffer* b : {&it->second.pairs, &it->second.masks, &it->second.g2, &it->second.raw}) dev_free(ctx, *b);
+        it = ctx->sel.erase(it);
+    }
+}
+
 si_status dev_alloc(si_ctx* ctx, DeviceBuffer& buf, size_t bytes) {
     dev_free(ctx, buf);
     if (bytes == 0) bytes = 16;
     bytes = (bytes + 255) & ~size_t(255);
-    if (ctx->used + bytes > ctx->budget) dev_free(ctx, ctx->bckpt);  // waits for the kernels that use it
+    if (ctx->used + bytes > ctx->budget) reclaim(ctx);
     if (ctx->used + bytes > ctx->budget)
         return fail(ctx, SI_ERR_BUDGET, "HBM budget exceeded: need " + std::to_string(bytes) + " more bytes, " +
                                             std::to_string(ctx->budget - ctx->used) + " left");
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && ctx->bckpt.ptr) {
+    if (e == cudaErrorMemoryAllocation && reclaimable_bytes(ctx)) {
         cudaGetLastError();
-        dev_free(ctx, ctx->bckpt);
+        reclaim(ctx);
         e = cudaMalloc(&p, bytes);
     }
     if (e != cudaSuccess) { cudaGetLastError(); return cuda_fail(ctx, e, "cudaMalloc"); }
@@ -106,6 +123,22 @@ void reset_index(si_ctx* ctx) {
     ctx->region_sel.clear();
     ctx->has_index = false;
     ctx->pbwt_flags = 0;
+}
+
+// Before the index of the same panel is built again: what it fills again with the
+// same sizes stays allocated (the head rows, the selection tables as stale ones).
+// Waits for the kernels that read them.
+si_status reuse_index(si_ctx* ctx) {
+    if (ctx->head.ptr || !ctx->sel.empty()) SI_CUDA(ctx, cudaDeviceSynchronize(), "index rebuild");
+    DeviceBuffer head = ctx->head;
+    ctx->head = DeviceBuffer{};
+    auto sel = std::move(ctx->sel);
+    ctx->sel.clear();
+    reset_index(ctx);
+    ctx->head = head;
+    ctx->sel = std::move(sel);
+    for (auto& kv : ctx->sel) kv.second.stale = true;
+    return SI_OK;
 }
 
 void clear_exceptions(si_ctx* ctx) {
@@ -217,7 +250,8 @@ si_status ensure_selection(si_ctx* ctx, uint32_t L, int kind, SelectionCache** o
             return fail(ctx, SI_ERR_INVALID_ARG, "bad selection kind");
     }
     auto& c = ctx->sel[{L, kind}];
-    if (!c.pairs.ptr || force) {
+    if (!c.pairs.ptr || force || c.stale) {
+        c.stale = false;  // no allocation may take it from here on
         c.L = L;
         c.kind = kind;
         if (!c.pairs.ptr) {
@@ -743,6 +777,7 @@ si_status si_ctx_destroy(si_ctx* ctx) {
     dev_free(ctx, ctx->trans);
     dev_free(ctx, ctx->ckpt);
     dev_free(ctx, ctx->bckpt);
+    dev_free(ctx, ctx->build);
     dev_free(ctx, ctx->smasks);
     dev_free(ctx, ctx->io_geno);
     dev_free(ctx, ctx->io_dosage);
@@ -780,7 +815,7 @@ const char* si_last_error(const si_ctx* ctx) { return ctx ? ctx->err.c_str() : "
 
 si_status si_ctx_memory(const si_ctx* ctx, uint64_t* used_bytes, uint64_t* budget_bytes) {
     if (!ctx) return SI_ERR_INVALID_ARG;
-    if (used_bytes) *used_bytes = ctx->used - ctx->bckpt.bytes;  // bckpt makes room for any other allocation
+    if (used_bytes) *used_bytes = ctx->used - reclaimable_bytes(ctx);
     if (budget_bytes) *budget_bytes = ctx->budget;
     return SI_OK;
 }
@@ -897,10 +932,10 @@ si_status si_pbwt_build(si_ctx* ctx, uint32_t flags) {
     if (!ctx) return SI_ERR_INVALID_ARG;
     if (!ctx->panel.ptr) return fail(ctx, SI_ERR_STATE, "no panel uploaded");
     SI_TRY(set_device(ctx));
-    reset_index(ctx);
+    SI_TRY(reuse_index(ctx));
     const uint32_t M = ctx->M, N = ctx->N;
-    SI_TRY(dev_alloc(ctx, ctx->head, (size_t)M * kHead * 4));
-    SI_CUDA(ctx, cudaMemsetAsync(ctx->head.ptr, 0, (size_t)M * kHead * 4, ctx->stream), "memset head");
+    if (!ctx->head.ptr) SI_TRY(dev_alloc(ctx, ctx->head, (size_t)M * kHead * 4));
+    if (N < kHead) SI_CUDA(ctx, cudaMemsetAsync(ctx->head.ptr, 0, (size_t)M * kHead * 4, ctx->stream), "memset head");
     if (flags & SI_PBWT_STORE_INDEX) SI_TRY(dev_alloc(ctx, ctx->prefix, (size_t)M * N * 4));
     if (flags & SI_PBWT_ROW_HASHES) {
         SI_TRY(dev_alloc(ctx, ctx->row_hash, (size_t)M * 8));
@@ -925,10 +960,16 @@ si_status si_pbwt_build(si_ctx* ctx, uint32_t flags) {
     const bool group_global = !sorted && S > 1 && pbwt_group_smem_bytes(N, ctx->W) > (size_t)max_optin;
     const size_t scratch_words = std::max<size_t>(sweep_global ? (size_t)2 * N * S : 0,
                                                   group_global ? (size_t)4 * N * (S - 1) : 0);
-    DeviceBuffer scratch, jobbuf, orders, gid, sortbuf;
-    si_status st = dev_alloc(ctx, jobbuf, S * sizeof(SweepJob));
-    if (st == SI_OK && scratch_words) st = dev_alloc(ctx, scratch, scratch_words * 4);
-    if (st == SI_OK && S > 1) st = dev_alloc(ctx, orders, sorted ? (size_t)(S - 1) * N * 8 : (size_t)S * N * 4);
+    DeviceBuffer scratch, gid, sortbuf;
+    si_status st = SI_OK;
+    if (scratch_words) st = dev_alloc(ctx, scratch, scratch_words * 4);
+    const size_t job_bytes = (S * sizeof(SweepJob) + 255) & ~size_t(255);
+    const size_t build_bytes = job_bytes + (S > 1 ? (sorted ? (size_t)(S - 1) * N * 8 : (size_t)S * N * 4) : 0);
+    if (st == SI_OK && ctx->build.bytes < build_bytes) st = dev_alloc(ctx, ctx->build, build_bytes);
+    // the buffer is this call's own until the sweep is through (no allocation below may reclaim it)
+    DeviceBuffer build = ctx->build;
+    ctx->build = DeviceBuffer{};
+    DeviceBuffer jobbuf{build.ptr, 0}, orders{(char*)build.ptr + job_bytes, 0};
     if (st == SI_OK && S > 1 && !sorted) st = dev_alloc(ctx, gid, (size_t)(S - 1) * N * 4);
     if (st == SI_OK && S > 1 && !sorted) st = dev_alloc(ctx, sortbuf, (size_t)4 * N * 4);
     cudaError_t e = cudaSuccess;
@@ -959,7 +1000,8 @@ si_status si_pbwt_build(si_ctx* ctx, uint32_t flags) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ctx->pbwt_ms, ctx->ev[0], ctx->ev[1]);
     }
-    for (DeviceBuffer* b : {&scratch, &jobbuf, &orders, &gid, &sortbuf}) dev_free(ctx, *b);
+    for (DeviceBuffer* b : {&scratch, &gid, &sortbuf}) dev_free(ctx, *b);
+    ctx->build = build;
     if (st != SI_OK) return st;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "PBWT sweep");
     ctx->has_index = true;

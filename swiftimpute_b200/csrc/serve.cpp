@@ -163,10 +163,10 @@ si_status pinned_reserve(Pinned& b, size_t bytes) {
 uint64_t reclaimable(const si_server* S, int k) {
     const si_ctx* c = S->ctx;
     const auto& z = S->slot[k];
-    uint64_t b = 0;
+    uint64_t b = si::reclaimable_bytes(c);
     for (const si::DeviceBuffer* x : {&c->t_counts, &c->t_segc, &c->t_aoff, &c->t_woff, &c->t_apos, &c->t_aem,
                                       &c->t_ckF, &c->t_ckB, &c->t_ckU, &c->job_regions,
-                                      &c->job_samples, &c->bckpt, &z.d_geno, &z.d_dos, &z.d_haps, &z.d_hp})
+                                      &c->job_samples, &z.d_geno, &z.d_dos, &z.d_haps, &z.d_hp})
         b += x->bytes;
     return b;
 }

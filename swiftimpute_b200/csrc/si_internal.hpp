@@ -75,6 +75,7 @@ struct SelectionCache {
     DeviceBuffer masks;  // [M] SlotMasks
     DeviceBuffer g2;     // [M][fb_lmax(L)] f32x2 non-zero alleles per slot at m and m + 1
     DeviceBuffer raw;    // [M][fb_lmax(L)][2] u8 allele bytes (panels with alleles other than 0/1 only)
+    bool stale = false;  // of an index since rebuilt: the buffers wait to be filled again, or make room
 };
 
 }  // namespace si
@@ -119,7 +120,9 @@ struct si_ctx {
     uint64_t trans_key = ~0ull;
     si::LinTrans trans0{1.f, 0.f};  // host copy of the first gap's transition
     si::DeviceBuffer ckpt;           // forward checkpoints (full-chain kernel)
-    si::DeviceBuffer bckpt;          // both directions' segment ends: held while the budget has room, freed for any other allocation
+    // Buffers kept between calls while the budget has room and freed for any other allocation (reclaim):
+    si::DeviceBuffer bckpt;          // both directions' segment ends (full-chain kernels)
+    si::DeviceBuffer build;          // start orders and jobs of the index build
     si::DeviceBuffer smasks;         // per-target slot masks [M][B] (target-aware selection)
     // typed-marker kernel scratch and tables
     si::DeviceBuffer t_counts, t_segc, t_aoff, t_woff, t_apos, t_aem, t_ckF, t_ckB, t_ckU;
@@ -148,6 +151,10 @@ struct si_ctx {
 
 namespace si {
 
+// Bytes the ctx holds only until another allocation needs them (counted in used),
+// and giving them up.
+uint64_t reclaimable_bytes(const si_ctx* ctx);
+void reclaim(si_ctx* ctx);
 // Allocation under the ctx's HBM budget.
 si_status dev_alloc(si_ctx* ctx, DeviceBuffer& buf, size_t bytes);
 void dev_free(si_ctx* ctx, DeviceBuffer& buf);

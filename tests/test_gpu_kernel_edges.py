@@ -177,3 +177,42 @@ def test_index_segments(engine, M, N_, p1):
     assert np.array_equal(engine.row_hashes(), hashes)
     if N_ <= 1025:
         assert np.array_equal(engine.prefix_rows(), oracle.pbwt_build(panel))
+
+
+def test_index_rebuilt_in_place():
+    """The same panel's index built again keeps its buffers: selections follow the build, imputation under
+    a new panel's index is the new one's, and kept buffers make room within the budget."""
+    from swiftimpute_b200.engine import Engine
+    M, N_ = 700, 600
+    panel, pos, _ = synth.make_panel(M, N_, 20, seed=3, spacing=1000)
+    other, _, _ = synth.make_panel(M, N_, 20, seed=4, spacing=1000)
+    codes, _, _ = synth.make_targets(panel, 40, synth.typed_every(M, 9), seed=5)
+    p = N.default_params(num_states=8, ne=20000)
+
+    def results(eng):
+        return eng.select_states(8), eng.select_states(4), eng.impute(codes, p, hap_prob=True)
+
+    with Engine(0) as eng:
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        first = results(eng)
+        peak = eng.memory()[0]
+        for _ in range(2):
+            eng.pbwt_build()
+            again = results(eng)
+            assert np.array_equal(first[0], again[0]) and np.array_equal(first[1], again[1])
+            for key in first[2]:
+                assert np.array_equal(first[2][key], again[2][key])
+        eng.impute(codes, N.default_params(num_states=8, ne=20000, flags=N.IMPUTE_FULL_CHAIN))
+        eng.upload_panel(other); eng.set_map(pos); eng.pbwt_build()
+        fresh = results(eng)
+    with Engine(0) as eng:
+        eng.upload_panel(other); eng.set_map(pos); eng.pbwt_build()
+        for a, b in zip(results(eng)[:2], fresh[:2]):
+            assert np.array_equal(a, b)
+    with Engine(0, hbm_budget_bytes=peak + (4 << 20)) as eng:  # the build's own scratch is 4 MB here at most
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        for L in (4, 8, 16, 32):
+            eng.select_states(L)
+        eng.pbwt_build(store_index=True)  # 1.7 MB of prefix rows beside what is kept
+        again = results(eng)
+        assert np.array_equal(first[0], again[0])
