@@ -58,6 +58,7 @@ struct TypedArgs {
     uint32_t K;                      // windows per posterior group (forward checkpoints every K windows)
     uint32_t stage;                  // posterior CTAs hold slot data in shared memory (set at its launch)
     uint32_t rows;                   // samples of a posterior warp (set at its launch)
+    uint32_t parts;                  // posterior warps that share a window group (a divisor of K, set at the launch)
     uint32_t max_windows;            // most windows of any sample (posterior grid)
     int sampling;
     float tie_eps;

@@ -829,8 +829,8 @@ __global__ void __launch_bounds__(kChainThreads, LM <= 16 ? 5 : 3) anchor_chain_
 // 20 for the floor), an anchor about 300. Launch times, one walk for all before
 // -> now: 10,000 x 50,000 (L = 8) 4.06 -> 2.35 ms (writing its 3 GB would take
 // 0.47); 2,003 x 30,011 0.76 -> 0.41; 4,000 x 20,000 (L = 16) 1.27 -> 0.68; 1,500
-// x 6,007 (L = 32, alleles only) 0.22 -> 0.18; one target x 1,644 98 -> 57 us;
-// 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 0.55 ms.
+// x 6,007 (L = 32, alleles only) 0.22 -> 0.18; one target x 1,644 98 -> 21 us;
+// 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 0.22 ms.
 
 // Lanes that take an anchor together, each lane by itself: 131 x 7,919 with sites of their own takes
 // 1.12 ms when a lane takes its anchors alone, 0.79 with 4, 0.83 with 8, 1.00 with 16.
@@ -1095,7 +1095,10 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
 
     // a warp takes A.rows samples (a divisor of 32): SW warps and SC CTAs of one window group
     const uint32_t SW = (A.B + A.rows - 1) / A.rows, SC = (SW + nw - 1) / nw;
-    const unsigned long long grp = blockIdx.x / SC;
+    // A.parts warps share a window group's windows; each carries alpha from the group's first anchor
+    const uint32_t Kp = K / A.parts;
+    const unsigned long long grp = blockIdx.x / SC / A.parts;
+    const unsigned long long first = grp * K + blockIdx.x / SC % A.parts * Kp;  // its first window
     const uint32_t w0cta = blockIdx.x % SC * nw;
     const uint32_t cta_threads = 32 * min(nw, SW - w0cta);  // the warps with samples
     if (w0cta + warp >= SW) return;  // whole warp
@@ -1103,14 +1106,14 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
     // a lane past the warp's samples or the batch's end repeats one of them, and writes nothing
     const bool real = lane < A.rows && row0 + lane < A.B;
     const uint32_t s = min(row0 + (lane & (A.rows - 1)), A.B - 1);
-    bool live = grp * K < A.max_windows;
+    bool live = first < A.max_windows;
     View v{};
     if (!kPlain) v = view_of(A, s);
     const uint32_t NA = A.counts[s];
     const unsigned long long ab = A.aoff[g] + (s & 31u), wb = A.woff[g] + (s & 31u);
     const uint32_t NW = (NA + C - 1) / C;
-    const uint32_t w0 = live ? (uint32_t)grp * K : 0u;
-    const uint32_t wend = min(w0 + K, NW);
+    const uint32_t w0 = live ? (uint32_t)first : 0u;
+    const uint32_t wend = min(w0 + Kp, NW);
     live = live && w0 < wend;
     const bool warp_live = __any_sync(kAll, live);
     if (!A.stage && !warp_live) return;  // whole warp
@@ -1156,9 +1159,21 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
             FL = make_float2(l, l);
         }
     };
+    // alpha over a run ({Q, S} = qs) and the emission em of the anchor at its end
+    auto alpha_step = [&](float2 qs, uint32_t em) {
+        float x[LM];
+#pragma unroll
+        for (int l = 0; l < LM; ++l) x[l] = a_of(l);
+        const float base = vsum<LM>(x) * qs.y;
+#pragma unroll
+        for (int l = 0; l < LM; ++l) x[l] = ((em >> l) & 1u) ? fmaf(qs.x, x[l], base) : 0.f;
+        const float inv = rcp_approx(vsum<LM>(x));
+#pragma unroll
+        for (int l = 0; l < LM; ++l) set_a(l, x[l] * inv);
+    };
     if (live) {
         stage_window<LM>(A, apos, aem, wb, NA, w0, st, lane);
-        const float4* src = reinterpret_cast<const float4*>(A.ckptF + (wb + 32ull * w0) * LM);
+        const float4* src = reinterpret_cast<const float4*>(A.ckptF + (wb + 32ull * grp * K) * LM);
         float x[LM];
 #pragma unroll
         for (uint32_t q = 0; q < Q4; ++q) {
@@ -1168,7 +1183,26 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
         const float inv = rcp_approx(vsum<LM>(x));
 #pragma unroll
         for (int l = 0; l < LM; ++l) set_a(l, x[l] * inv);
-        p0 = apos[32ull * w0 * C] & ~kShiftBit;
+        // alpha from the group's first anchor to this warp's
+        const uint32_t ka = (uint32_t)grp * K * C, kb = w0 * C;
+        uint32_t pa = apos[32ull * ka] & ~kShiftBit;
+        for (uint32_t k = ka; k < kb; k += 4) {
+            uint32_t pk[4], ek[4];
+            float2 qk[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {  // four anchors' loads together
+                const uint32_t kk = min(k + 1 + j, kb);
+                pk[j] = apos[32ull * kk] & ~kShiftBit;
+                ek[j] = aem[32ull * kk];
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) qk[j] = tabQS(tb, pk[j] - (j ? pk[j - 1] : pa));
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                if (k + 1 + j <= kb) alpha_step(qk[j], ek[j]);
+            pa = pk[3];
+        }
+        p0 = pa;
         mend = wend * C < NA ? (apos[32ull * wend * C] & ~kShiftBit) : len;
         m = p0;
         rebuild_window<LM>(A, tb, NA, len, w0, st, recW, recF, lane);
@@ -1366,15 +1400,7 @@ __global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
             rebuild_window<LM>(A, tb, NA, len, win, st, recW, recF, lane);
             if (win + 1 < wend) stage_window<LM>(A, apos, aem, wb, NA, win + 1, st, lane);
         }
-        float x[LM];
-#pragma unroll
-        for (int l = 0; l < LM; ++l) x[l] = a_of(l);
-        const float base = vsum<LM>(x) * qs.y;
-#pragma unroll
-        for (int l = 0; l < LM; ++l) x[l] = ((em >> l) & 1u) ? fmaf(qs.x, x[l], base) : 0.f;
-        const float inv = rcp_approx(vsum<LM>(x));
-#pragma unroll
-        for (int l = 0; l < LM; ++l) set_a(l, x[l] * inv);
+        alpha_step(qs, em);
         load_record(rec);
     };
 
@@ -1658,12 +1684,18 @@ cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
         if (e != cudaSuccess) return e;
     }
     const unsigned long long groups = ((unsigned long long)a.max_windows + a.K - 1) / a.K;
+    // A batch of few warps has several share a window group, while that leaves at most two a scheduler (the
+    // anchors before a warp's own cost it alpha steps alone): one target x 1,644 57 -> 21 us, 444 of them 60 ->
+    // 33, 131 x 7,919 with sites of their own 548 -> 224 (296 with at most one warp a scheduler).
+    f.parts = 1;
+    while (f.parts < 8 && a.K % (2 * f.parts) == 0 && groups * f.parts * 2 * typed_groups(a.B) <= 8u * 148u) f.parts *= 2;
+    const unsigned long long parts = groups * f.parts;
     // A batch of few warps gives each fewer samples, while that leaves at most two warps a scheduler:
     // lanes at their own sites wait for fewer others (131 x 7,919: 0.79 ms with 32 samples a warp, 0.58
     // with 8, 0.55 with 4, 0.75 with 2), and lanes in step lose nothing (444 x 1,644: 64 us and 60).
     f.rows = 32;
-    while (f.rows > 4 && groups * ((a.B + f.rows / 2 - 1) / (f.rows / 2)) <= 8u * 148u) f.rows /= 2;
-    const unsigned long long grid = groups * (((a.B + f.rows - 1) / f.rows + T / 32 - 1) / (T / 32));
+    while (f.rows > 4 && parts * ((a.B + f.rows / 2 - 1) / (f.rows / 2)) <= 8u * 148u) f.rows /= 2;
+    const unsigned long long grid = parts * (((a.B + f.rows - 1) / f.rows + T / 32 - 1) / (T / 32));
     if (grid == 0) return cudaSuccess;
     if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
     anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos><<<(uint32_t)grid, T, sm, s>>>(f);

@@ -216,3 +216,24 @@ def test_index_rebuilt_in_place():
         eng.pbwt_build(store_index=True)  # 1.7 MB of prefix rows beside what is kept
         again = results(eng)
         assert np.array_equal(first[0], again[0])
+
+
+# warps that share a window group (one target, a few) against one warp a group (many): the same bits, for
+# windows of any size
+@pytest.mark.parametrize("C", [1, 2, 3, 8])
+@pytest.mark.parametrize("L", [4, 8, 32])
+def test_window_parts(engine, C, L):
+    M = 1500
+    panel, pos, _ = synth.make_panel(M, 300, 20, seed=C, spacing=1000)
+    codes_all, _, _ = synth.make_targets(panel, 700, np.arange(M), seed=C + 1, het_range=(0.0, 1.0))
+    codes = own_sites(codes_all, np.random.default_rng(C).integers(300, M, 700), seed=C + 2)
+    codes[:64] = np.where(np.arange(M) % 3 == 0, codes_all[:64], 3)  # two groups on one array
+    engine.upload_panel(panel)
+    engine.set_map(pos)
+    engine.pbwt_build()
+    p = N.default_params(num_states=L, ne=20000, checkpoint_interval=C)
+    many = engine.impute(codes, p, hap_prob=True)
+    for rows in ([0], [5, 6, 7], list(range(60, 100)), [699]):
+        few = engine.impute(codes[rows], p, hap_prob=True)
+        for key in few:
+            assert np.array_equal(few[key], many[key][rows]), (key, rows)
