@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(kChainThreads, LM <= 16 ? 5 : 3) anchor_chain_
 // L = 8 (24 f32x2 operations for the slots, 15 for the sums, 47 for the argmax,
 // 20 for the floor), an anchor about 300. Launch times, one walk for all before
 // -> now: 10,000 x 50,000 (L = 8) 4.06 -> 2.35 ms (writing its 3 GB would take
-// 0.47); 2,003 x 30,011 0.76 -> 0.41; 4,000 x 20,000 (L = 16) 1.27 -> 0.68; 1,500
+// 0.47); 2,003 x 30,011 0.76 -> 0.41; 4,000 x 20,000 (L = 16) 1.27 -> 0.63; 1,500
 // x 6,007 (L = 32, alleles only) 0.22 -> 0.18; one target x 1,644 98 -> 21 us;
 // 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 0.22 ms.
 
@@ -1060,6 +1060,11 @@ __device__ __forceinline__ bool lanes_in_step(const TypedArgs& A, const View& v,
     return true;
 }
 
+// Warps an SM over registers: at L = 16 a plain batch runs 3 CTAs at 168 registers with a few
+// spills faster than 2 without (4,000 x 20,000: 668 -> 625 us).
+template <int LM, bool kPlain>
+constexpr int kPostCtas = LM <= 8 ? (kPlain ? 4 : 3) : LM == 16 && kPlain ? 3 : 2;
+
 // kFull: every sample of the launch uses all LM slots (no active-slot masking).
 // kFast: argmax picks, no P(hap=1). kPlain: every sample covers the whole
 // panel with the launch's one region (read from the kernel parameters).
@@ -1071,7 +1076,7 @@ __device__ __forceinline__ bool lanes_in_step(const TypedArgs& A, const View& v,
 // Tiles are aligned to absolute 32-marker columns, so a tile every lane of a
 // warp fills completely leaves as 128-bit row segments.
 template <int LM, bool kFull, bool kFast, bool kPlain, bool kDos>
-__global__ void __launch_bounds__(128, (LM <= 8 ? (kPlain ? 4 : 3) : 2))
+__global__ void __launch_bounds__(128, kPostCtas<LM, kPlain>)
     anchor_posterior_kernel(const __grid_constant__ TypedArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr uint32_t Q4 = LM / 4;
