@@ -161,6 +161,30 @@ def test_target_walk(engine, N_, M, B, L):
         assert np.array_equal(got[b], oracle.select_pairs_target(prefix, panel, codes[b], L)), b
 
 
+# a batch's last target beside lanes without one: its slots are its own walk's, not those of a target without
+# calls (what such a lane's codes read as), alone, at the end of a batch of any size and in the oracle
+@pytest.mark.parametrize("N_", [300, 1024, 10880])
+@pytest.mark.parametrize("B", [1, 2, 31, 33, 40, 63, 65])
+def test_target_walk_last_target(engine, N_, B):
+    M, L = 70, 8
+    panel, pos, _ = synth.make_panel(M, N_, 8, seed=B + N_)
+    codes = np.random.default_rng(B).choice(np.array([0, 2], np.uint8), (B, M))  # every marker typed, homozygous
+    engine.upload_panel(panel)
+    engine.set_map(pos)
+    engine.pbwt_build(store_index=True)
+    prefix = engine.prefix_rows()
+    want = oracle.select_pairs_target(prefix, panel, codes[-1], L)
+    none = oracle.select_pairs_target(prefix, panel, np.full(M, 3, np.uint8), L)
+    assert (want != none).any(axis=(1, 2)).mean() > 0.5  # the two walks part: a store of the other one would show
+    got = engine.select_states_target(L, codes)
+    assert np.array_equal(got[-1], want)
+    assert np.array_equal(engine.select_states_target(L, codes[-1:])[0], want)
+    p = N.default_params(num_states=L, ne=20000, selection_kind=N.SEL_TARGET)
+    batch, alone = engine.impute(codes, p, hap_prob=True), engine.impute(codes[-1:], p, hap_prob=True)
+    for key in batch:
+        assert np.array_equal(batch[key][-1], alone[key][0]), key
+
+
 # the index built from sorted segments (up to about 20,000 haplotypes) and from swept groups: segment counts
 # around powers of two, a last segment of any length, passes of eight markers with a remainder, many equal
 # haplotypes (long groups) and none
