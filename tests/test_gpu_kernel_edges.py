@@ -112,6 +112,42 @@ def test_posterior_walks(engine, L, M, every, B, spacing, other_alleles):
                     assert np.array_equal(alone[key], beside[key][0::2]), (key, kw, out)
 
 
+# runs longer than the run tables (4,096 markers) in the walk in step, two cells a step by the closed form: the
+# oracle's, and bit for bit the lanes' own walk's
+@pytest.mark.parametrize("L,M,every,B", [(4, 4099, 4099, 1), (3, 8400, 4097, 33), (8, 13001, 4333, 5), (16, 9000, 4500, 32),
+                                         (32, 8777, 4388, 7)])
+@pytest.mark.parametrize("spacing", [1000, 500_000])
+def test_long_runs_in_step(engine, L, M, every, B, spacing):
+    panel, pos, _ = synth.make_panel(M, 64, 8, seed=M + L, spacing=spacing)
+    codes, _, _ = synth.make_targets(panel, B, synth.typed_every(M, every), seed=M + 1, het_range=(0.0, 1.0))
+    check(engine, panel, pos, codes, L)
+    mixed = np.repeat(codes, 2, axis=0)  # an extra site in every other row: the lanes of a warp are not in step
+    mixed[1::2, M // 3] = 1
+    for kw in ({}, {"sampling": N.SAMPLE_PHILOX}):
+        for out in ({"hap_prob": True}, {}, {"dosage": False}):
+            p = N.default_params(num_states=L, ne=20000, **kw)
+            alone, beside = engine.impute(codes, p, **out), engine.impute(mixed, p, **out)
+            for key in alone:
+                if key != "haps" or not kw:  # a draw is keyed by the row's sample id
+                    assert np.array_equal(alone[key], beside[key][0::2]), (key, kw, out)
+
+
+def test_long_runs_in_step_time(engine):
+    M, B = 9100, 32
+    panel, pos, _ = synth.make_panel(M, 64, 8, seed=1, spacing=1000)
+    engine.upload_panel(panel)
+    engine.set_map(pos)
+    engine.pbwt_build()
+    p = N.default_params(num_states=8, ne=20000)
+
+    def posterior_ms(every):
+        codes, _, _ = synth.make_targets(panel, B, synth.typed_every(M, every), seed=2)
+        return min((engine.impute(codes, p), engine.last_kernel_ms()[3])[1] for _ in range(5))
+
+    # the same markers in runs past the tables and within them: 3.24 and 1.69 ms (5.83 with a cell a step)
+    assert posterior_ms(4500) <= 2.6 * posterior_ms(4000)
+
+
 # the full chain in parallel segments against the oracle and against one pass over the chain (the
 # kernel that a budget without room for the segments' ends falls back to):
 # lengths around the checkpoint segments, the staged blocks (8, 4) and code chunks (32), B around a warp
