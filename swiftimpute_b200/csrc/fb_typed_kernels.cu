@@ -832,10 +832,6 @@ __global__ void __launch_bounds__(kChainThreads, LM <= 16 ? 5 : 3) anchor_chain_
 // x 6,007 (L = 32, alleles only) 0.22 -> 0.18; one target x 1,644 98 -> 21 us;
 // 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 0.22 ms.
 
-// Lanes that take an anchor together, each lane by itself: 131 x 7,919 with sites of their own takes
-// 1.12 ms when a lane takes its anchors alone, 0.79 with 4, 0.83 with 8, 1.00 with 16.
-constexpr int kTurn = 4;
-
 // high word of farg' for a uniform run and for a negligible floor
 constexpr uint32_t kInfHi = 0x7ff00000u;
 constexpr uint32_t kNegInfHi = 0xfff00000u;
@@ -1649,9 +1645,10 @@ __global__ void __launch_bounds__(128, kPostCtas<LM, kPlain>)
         return;
     }
 
-    // ---- every lane by itself: lanes reach their anchors at different cells, and an anchor costs about
-    // three steps of cells, so those at one wait until kTurn of them (or all that still have cells in the
-    // tile) are there and take it together.
+    // ---- every lane by itself: lanes reach their anchors at different cells. Those at one take it at once,
+    // then all lanes step. (Lanes that waited at an anchor until four of them were there, or none had cells left
+    // in the tile, made the others' wait shorter but left the tile's last cells to few lanes: 9,000 x 6,000, L = 8,
+    // whole calls, a site every 11 markers 2.23 ms against 2.21, every 40 2.35 against 2.22, every 200 4.57 against 3.54.)
     uint32_t tbase = m & ~31u;
     for (;;) {
         const bool on = live && m < mend;
@@ -1659,16 +1656,15 @@ __global__ void __launch_bounds__(128, kPostCtas<LM, kPlain>)
         const uint32_t tend = min(tbase + 32, mend), tlo = on ? m - tbase : 32u;
         for (;;) {
             const bool more = on && m < tend, turn = more && m == p1;
-            const uint32_t turns = __ballot_sync(kAll, turn), steps = __ballot_sync(kAll, more && !turn);
-            if (!(turns | steps)) break;
-            if (!steps || __popc(turns) >= kTurn) {
-                if (turn) {
-                    anchor(tabQS(tb, p1 - p0));
-                    p0 = p1;
-                    p1 = fr.z;
-                    in_tab = p1 - p0 < tb.NT;
-                }
-            } else if (more && !turn) {  // the next cells of the run, two per step when they pair up
+            if (!__any_sync(kAll, more)) break;
+            if (turn) {
+                anchor(tabQS(tb, p1 - p0));
+                p0 = p1;
+                p1 = fr.z;
+                in_tab = p1 - p0 < tb.NT;
+            }
+            __syncwarp();
+            if (more) {  // the next cells of the run, two per step when they pair up
                 const uint32_t e = min(p1, tend);
                 const bool two = (m & 1u) == 0u && m + 1 < e;
                 float4 qa, qb;
@@ -1707,8 +1703,9 @@ cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
     while (f.parts < 8 && a.K % (2 * f.parts) == 0 && groups * f.parts * 2 * typed_groups(a.B) <= 8u * 148u) f.parts *= 2;
     const unsigned long long parts = groups * f.parts;
     // A batch of few warps gives each fewer samples, while that leaves at most two warps a scheduler:
-    // lanes at their own sites wait for fewer others (131 x 7,919: 0.79 ms with 32 samples a warp, 0.58
-    // with 8, 0.55 with 4, 0.75 with 2), and lanes in step lose nothing (444 x 1,644: 64 us and 60).
+    // lanes at their own sites wait for fewer others (131 x 7,919, a window group a warp: 0.79 ms with 32
+    // samples a warp, 0.58 with 8, 0.55 with 4, 0.75 with 2), and lanes in step lose nothing (444 x 1,644: 64
+    // us and 60).
     f.rows = 32;
     while (f.rows > 4 && parts * ((a.B + f.rows / 2 - 1) / (f.rows / 2)) <= 8u * 148u) f.rows /= 2;
     const unsigned long long grid = parts * (((a.B + f.rows - 1) / f.rows + T / 32 - 1) / (T / 32));
