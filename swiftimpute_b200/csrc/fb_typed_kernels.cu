@@ -1056,8 +1056,8 @@ __device__ __forceinline__ bool lanes_in_step(const TypedArgs& A, const View& v,
     return true;
 }
 
-// Warps an SM over registers: at L = 16 a plain batch runs 3 CTAs at 168 registers with a few
-// spills faster than 2 without (4,000 x 20,000: 668 -> 625 us).
+// Warps an SM over registers: at L = 16 a plain batch runs 3 CTAs at 168 registers faster than
+// 2 (4,000 x 20,000: 668 -> 625 us; launch_post_v has the exception).
 template <int LM, bool kPlain>
 constexpr int kPostCtas = LM <= 8 ? (kPlain ? 4 : 3) : LM == 16 && kPlain ? 3 : 2;
 
@@ -1071,8 +1071,8 @@ constexpr int kPostCtas = LM <= 8 ? (kPlain ? 4 : 3) : LM == 16 && kPlain ? 3 : 
 // marker or last marker takes a step alone (the second half is discarded).
 // Tiles are aligned to absolute 32-marker columns, so a tile every lane of a
 // warp fills completely leaves as 128-bit row segments.
-template <int LM, bool kFull, bool kFast, bool kPlain, bool kDos>
-__global__ void __launch_bounds__(128, kPostCtas<LM, kPlain>)
+template <int LM, bool kFull, bool kFast, bool kPlain, bool kDos, int kCtas>
+__global__ void __launch_bounds__(128, kCtas)
     anchor_posterior_kernel(const __grid_constant__ TypedArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr uint32_t Q4 = LM / 4;
@@ -1686,15 +1686,6 @@ cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
     TypedArgs f = a;
     f.stage = sm + post_cta_bytes(LM, kDos) <= 227u * 1024u;
     if (f.stage) sm += post_cta_bytes(LM, kDos);
-    // set outside stream capture only (a plan launches once before it is captured)
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaError_t e = cudaStreamIsCapturing(s, &cs);
-    if (e != cudaSuccess) return e;
-    if (cs == cudaStreamCaptureStatusNone) {
-        e = cudaFuncSetAttribute(anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-    }
     const unsigned long long groups = ((unsigned long long)a.max_windows + a.K - 1) / a.K;
     // A batch of few warps has several share a window group, while that leaves at most two a scheduler (the
     // anchors before a warp's own cost it alpha steps alone): one target x 1,644 57 -> 21 us, 444 of them 60 ->
@@ -1711,8 +1702,27 @@ cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
     const unsigned long long grid = parts * (((a.B + f.rows - 1) / f.rows + T / 32 - 1) / (T / 32));
     if (grid == 0) return cudaSuccess;
     if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-    anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos><<<(uint32_t)grid, T, sm, s>>>(f);
-    return cudaGetLastError();
+    auto launch = [&](auto kernel) -> cudaError_t {
+        // set outside stream capture only (a plan launches once before it is captured)
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(s, &cs);
+        if (e != cudaSuccess) return e;
+        if (cs == cudaStreamCaptureStatusNone) {
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            if (e != cudaSuccess) return e;
+        }
+        kernel<<<(uint32_t)grid, T, sm, s>>>(f);
+        return cudaGetLastError();
+    };
+    // With 16 slots, argmax and dosage the third CTA's register bound spills. In step the CTA is worth it (3,000 x
+    // 20,000, whole calls: 0.87 -> 0.82 ms); lanes by themselves wait for memory, which more warps do not hide (9,000 x
+    // 6,000 with sites of their own, every 25 markers 2.79 -> 3.65 ms, every 60 2.84 -> 3.75, 131 targets 0.31 -> 0.35).
+    // Samples of one array have equally long lists: three where every group's longest list is the batch's longest and
+    // there are CTAs for it, else two.
+    if constexpr (LM == 16 && kFull && kPlain && kFast && kDos)
+        if (grid <= 2u * 148u || a.total_windows != 32ull * typed_groups(a.B) * a.max_windows)
+            return launch(anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos, 2>);
+    return launch(anchor_posterior_kernel<LM, kFull, kFast, kPlain, kDos, kPostCtas<LM, kPlain>>);
 }
 
 template <int LM, bool kFull>

@@ -297,3 +297,22 @@ def test_window_parts(engine, C, L):
         few = engine.impute(codes[rows], p, hap_prob=True)
         for key in few:
             assert np.array_equal(few[key], many[key][rows]), (key, rows)
+
+
+# L = 16: three CTAs an SM for a large batch, two for a small one: the oracle's, and the same bits in both
+@pytest.mark.parametrize("L", [12, 16])
+@pytest.mark.parametrize("own", [False, True])
+def test_third_cta(engine, L, own):
+    M, B = 2000, 5000  # 1,250 CTAs
+    panel, pos, _ = synth.make_panel(M, 200, 12, seed=L, spacing=1000)
+    codes_all, _, _ = synth.make_targets(panel, 40, np.arange(M), seed=L + 1, het_range=(0.0, 1.0))
+    few = np.where(np.arange(M) % 8 == 0, codes_all, 3).astype(np.uint8)
+    if own:
+        few = own_sites(codes_all, np.random.default_rng(L).integers(100, 400, 40), seed=L + 2)
+    check(engine, panel, pos, few, L)
+    many = few[np.arange(B) % 40]
+    for kw, out in (({}, {}), ({}, {"dosage": False}), ({"sampling": N.SAMPLE_PHILOX}, {"hap_prob": True, "haps": False})):
+        p = N.default_params(num_states=L, ne=20000, **kw)
+        a, b = engine.impute(few, p, **out), engine.impute(many, p, **out)
+        for key in a:
+            assert np.array_equal(a[key][np.arange(B) % 40], b[key]), (key, kw)
