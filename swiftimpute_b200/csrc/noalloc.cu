@@ -80,7 +80,8 @@ extern "C" si_status si_impute_device_noalloc(si_ctx* ctx, const si_impute_param
     int kind = p->selection_kind;
     if (kind == SI_SEL_AUTO) kind = (L <= 32 && ctx->N <= 10000) ? SI_SEL_WARP : SI_SEL_INSERTION;
     auto it = ctx->sel.find({L, kind});
-    if (it == ctx->sel.end() || !it->second.masks.ptr || !ctx->trans.ptr || ctx->trans_key != trans_key_of(p))
+    if (it == ctx->sel.end() || it->second.stale || !it->second.masks.ptr || !ctx->trans.ptr ||
+        ctx->trans_key != trans_key_of(p))
         return fail(ctx, SI_ERR_STATE,
                     "set-up missing: run si_impute or si_impute_device once with the same parameters first "
                     "(that call allocates the slot and transition tables)");

@@ -1,0 +1,60 @@
+"""What a context keeps between calls: tables of an index since rebuilt, buffers
+under a tight budget, calls that failed half way (B200 only).
+"""
+from ctypes import byref, c_void_p
+
+import numpy as np
+import pytest
+
+from swiftimpute_b200 import _native as N
+from swiftimpute_b200 import synth
+from swiftimpute_b200.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+ERR_STATE, ERR_BUDGET = 5, 7
+
+
+def noalloc(torch, eng, codes, p):
+    """si_impute_device_noalloc: its status and the dosage it wrote."""
+    g = torch.from_numpy(codes).cuda()
+    dos = torch.zeros(codes.shape, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    st = eng.lib.si_impute_device_noalloc(eng.h, byref(p), c_void_p(g.data_ptr()), codes.shape[0],
+                                          c_void_p(dos.data_ptr()), None, None, None)
+    torch.cuda.synchronize()
+    return st, dos.cpu().numpy()
+
+
+def small(seed=1, M=600, N_=300, B=16):
+    panel, pos, _ = synth.make_panel(M, N_, 12, seed=seed, spacing=100)
+    codes, _, _ = synth.make_targets(panel, B, synth.typed_every(M, 5), seed=seed + 1)
+    return panel, pos, codes
+
+
+@pytest.mark.parametrize("kind", [N.SEL_AUTO, N.SEL_FIRST_PAIRS])
+def test_noalloc_after_a_rebuild(kind):
+    """Tables of an index since rebuilt, or whose rebuild failed, are not set-up: the call is refused until an
+    allocating call has filled them."""
+    torch = pytest.importorskip("torch")
+    panel, pos, codes = small()
+    M, N_ = panel.shape
+    p = N.default_params(num_states=8, ne=10000, selection_kind=kind)
+    with Engine(0) as eng:
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        eng.impute(codes, p)
+        st, first = noalloc(torch, eng, codes, p)
+        assert st == N.SI_OK
+        eng.pbwt_build()
+        assert noalloc(torch, eng, codes, p)[0] == ERR_STATE
+        eng.impute(codes, p)
+        st, again = noalloc(torch, eng, codes, p)
+        assert st == N.SI_OK and np.array_equal(first, again)
+        used = eng.memory()[0]
+    with Engine(0, hbm_budget_bytes=used + M * N_ * 2) as eng:  # no room for prefix rows
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        eng.impute(codes, p)
+        assert noalloc(torch, eng, codes, p)[0] == N.SI_OK
+        with pytest.raises(N.SIError):
+            eng.pbwt_build(store_index=True)
+        assert noalloc(torch, eng, codes, p)[0] == ERR_STATE
