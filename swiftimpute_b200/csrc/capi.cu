@@ -249,25 +249,41 @@ si_status ensure_selection(si_ctx* ctx, uint32_t L, int kind, SelectionCache** o
         if (kind != SI_SEL_WARP && kind != SI_SEL_INSERTION)
             return fail(ctx, SI_ERR_INVALID_ARG, "bad selection kind");
     }
-    auto& c = ctx->sel[{L, kind}];
-    if (!c.pairs.ptr || force || c.stale) {
-        c.stale = false;  // no allocation may take it from here on
-        c.L = L;
-        c.kind = kind;
-        if (!c.pairs.ptr) {
-            SI_TRY(dev_alloc(ctx, c.pairs, (size_t)ctx->M * L * 2 * sizeof(uint32_t)));
-            SI_TRY(dev_alloc(ctx, c.masks, (size_t)ctx->M * sizeof(SlotMasks)));
-            SI_TRY(dev_alloc(ctx, c.g2, (size_t)ctx->M * fb_lmax(L) * sizeof(float2)));
-            if (ctx->n_ex) SI_TRY(dev_alloc(ctx, c.raw, (size_t)ctx->M * fb_lmax(L) * 2));
-        }
-        SI_CUDA(ctx,
-                launch_select((const uint32_t*)ctx->head.ptr, (const uint32_t*)ctx->panel.ptr, ctx->M, ctx->N, ctx->W,
-                              L, kind, (const unsigned long long*)ctx->ex_off.ptr, (const uint32_t*)ctx->ex_ent.ptr,
-                              (uint32_t*)c.pairs.ptr, (SlotMasks*)c.masks.ptr, (float2*)c.g2.ptr, (uint8_t*)c.raw.ptr,
-                              fb_lmax(L), s ? s : ctx->stream),
-                "select kernel");
+    const auto key = std::make_pair(L, kind);
+    const auto it = ctx->sel.find(key);
+    if (it != ctx->sel.end() && !it->second.stale && !force) {
+        *out = &it->second;
+        return SI_OK;
     }
-    *out = &c;
+    // The entry is out of the cache while it is filled: no allocation below can reclaim its buffers, and one
+    // that fails half way leaves none behind (an entry in the cache that is not stale is whole).
+    SelectionCache c;
+    if (it != ctx->sel.end()) {
+        c = it->second;
+        ctx->sel.erase(it);
+    }
+    c.L = L;
+    c.kind = kind;
+    c.stale = false;
+    si_status st = SI_OK;
+    if (!c.pairs.ptr) {
+        st = dev_alloc(ctx, c.pairs, (size_t)ctx->M * L * 2 * sizeof(uint32_t));
+        if (st == SI_OK) st = dev_alloc(ctx, c.masks, (size_t)ctx->M * sizeof(SlotMasks));
+        if (st == SI_OK) st = dev_alloc(ctx, c.g2, (size_t)ctx->M * fb_lmax(L) * sizeof(float2));
+        if (st == SI_OK && ctx->n_ex) st = dev_alloc(ctx, c.raw, (size_t)ctx->M * fb_lmax(L) * 2);
+    }
+    if (st == SI_OK) {
+        const cudaError_t e = launch_select(
+            (const uint32_t*)ctx->head.ptr, (const uint32_t*)ctx->panel.ptr, ctx->M, ctx->N, ctx->W, L, kind,
+            (const unsigned long long*)ctx->ex_off.ptr, (const uint32_t*)ctx->ex_ent.ptr, (uint32_t*)c.pairs.ptr,
+            (SlotMasks*)c.masks.ptr, (float2*)c.g2.ptr, (uint8_t*)c.raw.ptr, fb_lmax(L), s ? s : ctx->stream);
+        if (e != cudaSuccess) st = cuda_fail(ctx, e, "select kernel");
+    }
+    if (st != SI_OK) {
+        for (DeviceBuffer* b : {&c.pairs, &c.masks, &c.g2, &c.raw}) dev_free(ctx, *b);
+        return st;
+    }
+    *out = &(ctx->sel[key] = c);
     return SI_OK;
 }
 

@@ -58,3 +58,42 @@ def test_noalloc_after_a_rebuild(kind):
         with pytest.raises(N.SIError):
             eng.pbwt_build(store_index=True)
         assert noalloc(torch, eng, codes, p)[0] == ERR_STATE
+
+
+@pytest.mark.parametrize("room", ["pairs", "masks", "weights"])
+def test_selection_that_does_not_fit(room):
+    """A selection whose tables run out of budget half way is refused every time it is asked for, after a rebuild
+    of the index too, holds nothing, and is right once there is room."""
+    L = 16
+    panel, pos, codes = small(seed=3, M=3000, N_=100, B=4)
+    if room == "weights":  # the last table: allele bytes of a panel with others than 0 and 1
+        panel = panel.copy()
+        panel[::7, ::5] = 255
+    M = panel.shape[0]
+
+    def up(nbytes):
+        return -(-nbytes // 256) * 256
+
+    parts = [up(M * L * 8), up(M * 16), up(M * L * 8)]  # pairs, masks, weights
+    with Engine(0) as eng:
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        base = eng.memory()[0]
+        want = eng.select_states(L)
+        whole = eng.memory()[0] - base
+    have = sum(parts[:["pairs", "masks", "weights"].index(room) + 1])
+    assert have < whole
+    with Engine(0, hbm_budget_bytes=base + have + 256) as eng:
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        for rebuild in (False, False, True, False):
+            if rebuild:
+                eng.pbwt_build()
+            with pytest.raises(N.SIError) as e:
+                eng.select_states(L)
+            assert e.value.status == ERR_BUDGET
+            assert eng.memory()[0] == base
+        assert np.array_equal(eng.select_states(1)[:, 0], want[:, 0])  # what fits beside it is served
+    with Engine(0, hbm_budget_bytes=base + whole) as eng:
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        for _ in range(2):
+            assert np.array_equal(eng.select_states(L), want)
+            eng.pbwt_build()
