@@ -571,7 +571,7 @@ size_t smem_bytes(uint32_t T, uint32_t C, bool hprob = true) {
 
 template <int LM, bool kAll>
 cudaError_t launch_segments(const FbArgs& fa, uint32_t T, size_t sm, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(fb_segment_kernel<LM, kAll>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(fb_segment_kernel<LM, kAll>);
     if (e != cudaSuccess) return e;
     const unsigned long long grid = (unsigned long long)((fa.B + T - 1) / T) * (kAll ? 1u : fa.nseg);
     if (grid > 0x7fffffffull) return cudaErrorInvalidConfiguration;
@@ -582,7 +582,7 @@ cudaError_t launch_segments(const FbArgs& fa, uint32_t T, size_t sm, cudaStream_
 template <int LM>
 cudaError_t launch_lm(const FbArgs& fa, uint32_t T, cudaStream_t s) {
     const size_t sm = smem_bytes<LM>(T, fa.C, fa.hprob != nullptr);
-    if (sm > 227u * 1024u) return cudaErrorInvalidValue;
+    if (sm > kMaxSmem) return cudaErrorInvalidValue;
     if (!fa.bckpt) return launch_segments<LM, true>(fa, T, sm, s);
     const uint32_t ctas = 2 * ((fa.B + 31) / 32);
     if (fa.L == LM) fb_ends_kernel<LM, true><<<ctas, kEndsThreads, 0, s>>>(fa);

@@ -1708,7 +1708,7 @@ cudaError_t launch_post_v(const TypedArgs& a, cudaStream_t s) {
         cudaError_t e = cudaStreamIsCapturing(s, &cs);
         if (e != cudaSuccess) return e;
         if (cs == cudaStreamCaptureStatusNone) {
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            e = allow_smem(kernel);
             if (e != cudaSuccess) return e;
         }
         kernel<<<(uint32_t)grid, T, sm, s>>>(f);

@@ -662,7 +662,7 @@ cudaError_t launch_pbwt_sweep(const uint32_t* d_panel, const SweepJob* d_jobs, u
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const size_t full = pbwt_sweep_smem_bytes(N, W);
     auto go = [&](auto kernel, size_t smem, uint32_t* gp) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(kernel);
         if (e != cudaSuccess) return e;
         kernel<<<n_jobs, T, smem, s>>>(d_panel, d_jobs, N, W, E, d_init, d_init16, d_head, d_prefix, d_hash, gp);
         return cudaSuccess;
@@ -694,10 +694,11 @@ cudaError_t launch_pbwt_orders(const uint32_t* d_panel, const SweepJob* d_jobs, 
                                uint16_t* d_buf, const uint16_t** d_orders, cudaStream_t s) {
     const size_t sm = pbwt_sort_smem_bytes(N, W), words = (size_t)n_jobs * N;
     uint16_t *o = d_buf, *r = o + words, *o2 = r + words, *r2 = o2 + words;
-    cudaError_t e = cudaFuncSetAttribute(pbwt_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(pbwt_double_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(pbwt_rank_kernel);
+    if (e == cudaSuccess) e = allow_smem(pbwt_double_kernel);
     if (e != cudaSuccess) return e;
     pbwt_rank_kernel<<<n_jobs, kSortThreads, sm, s>>>(d_panel, d_jobs, N, W, o, r);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;  // the rounds index by what it wrote
     const uint32_t bits = N > 1 ? 32u - (uint32_t)__builtin_clz(N - 1) : 0u;  // ranks are < N
     for (uint32_t d = 1; d < n_jobs; d *= 2) {
         pbwt_double_kernel<<<n_jobs, kSortThreads, sm, s>>>(o, r, N, d, bits, o2, r2);
@@ -721,11 +722,11 @@ cudaError_t launch_pbwt_groups(const uint32_t* d_panel, const SweepJob* d_jobs, 
     const size_t full = pbwt_group_smem_bytes(N, W);
     cudaError_t e;
     if (full <= (size_t)max_optin) {
-        e = cudaFuncSetAttribute(pbwt_group_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)full);
+        e = allow_smem(pbwt_group_kernel<true>);
         if (e == cudaSuccess) pbwt_group_kernel<true><<<n_jobs, T, full, s>>>(d_panel, d_jobs, N, W, E, d_gid, nullptr);
     } else {
         const size_t small = (size_t)(2 * W + 2 * 5 * 32) * 4;
-        e = cudaFuncSetAttribute(pbwt_group_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small);
+        e = allow_smem(pbwt_group_kernel<false>);
         if (e == cudaSuccess)
             pbwt_group_kernel<false><<<n_jobs, T, small, s>>>(d_panel, d_jobs, N, W, E, d_gid, d_scratch);
     }

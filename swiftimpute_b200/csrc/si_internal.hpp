@@ -169,6 +169,15 @@ si_status cuda_fail(si_ctx* ctx, cudaError_t e, const char* what);
 // threads other than the ctx's user may call it.
 bool region_first_gap_ok(const si_ctx* ctx, const si_impute_params* p, uint32_t m_begin, uint32_t m_end);
 
+// Dynamic shared memory of a CTA at most.
+constexpr size_t kMaxSmem = 227u * 1024u;
+// Lets kernel launch with up to kMaxSmem. The limit belongs to the function on its device, so it is the
+// same at every launch: one fitted to the launch could be lowered by another thread's context before it.
+template <class Kernel>
+cudaError_t allow_smem(Kernel kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+}
+
 // Kernel launchers (pbwt_kernels.cu, select_kernels.cu, fb_kernels.cu).
 cudaError_t launch_pack_panel(const uint8_t* d_u8, uint32_t M, uint32_t N, uint32_t W, uint32_t* d_words,
                               cudaStream_t s);

@@ -1,6 +1,7 @@
 """What a context keeps between calls: tables of an index since rebuilt, buffers
 under a tight budget, calls that failed half way (B200 only).
 """
+import threading
 from ctypes import byref, c_void_p
 
 import numpy as np
@@ -97,3 +98,65 @@ def test_selection_that_does_not_fit(room):
         for _ in range(2):
             assert np.array_equal(eng.select_states(L), want)
             eng.pbwt_build()
+
+
+def run_threads(works):
+    """Each callable 1,000 times in a thread of its own; the first exception is raised here."""
+    failed = []
+
+    def loop(work):
+        try:
+            for _ in range(1000):
+                work()
+        except Exception as x:
+            failed.append(x)
+
+    threads = [threading.Thread(target=loop, args=(w,)) for w in works]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    if failed:
+        raise failed[0]
+
+
+def test_imputations_in_two_threads():
+    """A context each in two threads of a device, their kernels launched with different amounts of shared memory
+    (outputs, checkpoint sizes): every call succeeds and is the same as alone."""
+    panel, pos, codes = small(seed=5, M=60, N_=64, B=2)
+
+    def params(C, flags=0):
+        return N.default_params(num_states=8, ne=20000, flags=flags, checkpoint_interval=C, block_threads=128)
+
+    chain = N.IMPUTE_FULL_CHAIN
+    calls = [[(params(32, chain), True), (params(32, chain), False), (params(12), False)],
+             [(params(8, chain), True), (params(8, chain), False), (params(2), False)]]
+    with Engine(0) as one, Engine(0) as other:
+        works = []
+        for e, mine in zip((one, other), calls):
+            e.upload_panel(panel); e.set_map(pos); e.pbwt_build()
+            alone = [e.impute(codes, p, hap_prob=hp) for p, hp in mine]
+
+            def work(e=e, mine=mine, alone=alone):
+                for (p, hp), want in zip(mine, alone):
+                    got = e.impute(codes, p, hap_prob=hp)
+                    assert all(np.array_equal(got[k], want[k]) for k in want)
+
+            works.append(work)
+        run_threads(works)
+
+
+def test_index_builds_in_two_threads():
+    with Engine(0) as one, Engine(0) as other:
+        works = []
+        for e, N_ in ((one, 400), (other, 6000)):
+            panel, _, _ = synth.make_panel(130, N_, 8, seed=N_)
+            e.upload_panel(panel); e.pbwt_build()
+            alone = e.select_states(8)
+
+            def work(e=e, alone=alone):
+                e.pbwt_build()
+                assert np.array_equal(e.select_states(8), alone)
+
+            works.append(work)
+        run_threads(works)
