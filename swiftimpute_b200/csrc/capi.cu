@@ -540,8 +540,8 @@ si_status run_device(si_ctx* ctx, const si_impute_params* p, const uint8_t* d_ge
         const size_t ends = (fb_ckpt_bytes(B, ctx->M, p->num_states, c) + 255) & ~size_t(255);
         const size_t need = ends + fb_back_bytes(B, ctx->M, p->num_states, c);
         if (ctx->bckpt.bytes < need) {
-            dev_free(ctx, ctx->bckpt);
-            if (ctx->used + need + 255 > ctx->budget) continue;
+            // room beside what an allocation does not reclaim; the ends held now stay where a size does not fit
+            if (ctx->used - reclaimable_bytes(ctx) + need + 255 > ctx->budget) continue;
             if (dev_alloc(ctx, ctx->bckpt, need) != SI_OK) continue;
         }
         C = c;

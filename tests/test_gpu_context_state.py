@@ -160,3 +160,84 @@ def test_index_builds_in_two_threads():
 
             works.append(work)
         run_threads(works)
+
+
+def ends_bytes(B, M, lmax, C):
+    """The full chain's ends at segments of C markers: alpha's, a 256-byte boundary, beta's and their units."""
+    n = max(-(-M // C) - 1, 1)
+    return -(-n * lmax * B * 4 // 256) * 256 + n * (lmax * 4 + 8) * B
+
+
+def test_full_chain_makes_room_for_its_ends():
+    """Under a budget whose room is held by tables of an index since rebuilt, the full chain's segments still run
+    in parallel: the tables make room, and no one-pass checkpoints (which would count as used) are allocated."""
+    panel, pos, codes = small(seed=7, M=1000, N_=64, B=500)
+    chain = N.default_params(num_states=8, ne=20000, flags=N.IMPUTE_FULL_CHAIN)
+
+    def before(eng):
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build()
+        eng.impute(codes, N.default_params(num_states=8, ne=20000))
+        for L in range(9, 33):
+            eng.select_states(L)
+        full = eng.memory()[0]
+        eng.pbwt_build()
+        return full
+
+    with Engine(0) as wide:
+        full = before(wide)
+        assert full - wide.memory()[0] > ends_bytes(500, 1000, 8, 16)  # the tables that wait
+        want = wide.impute(codes, chain)
+        used = wide.memory()[0]
+    with Engine(0, hbm_budget_bytes=full + (64 << 10)) as tight:
+        before(tight)
+        got = tight.impute(codes, chain)
+        assert tight.memory()[0] == used
+    for key in want:
+        assert np.array_equal(got[key], want[key])
+
+
+def device_call(torch, eng, codes, p):
+    """A full-chain call on device buffers of a stream of its own, warmed up: (stream, dosage, the call)."""
+    g = torch.from_numpy(codes).cuda()
+    dos = torch.zeros(codes.shape, dtype=torch.float32, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def call():
+        eng.impute_device(g.data_ptr(), codes.shape[0], p, dos.data_ptr(), None, None, stream=stream.cuda_stream)
+
+    call()
+    torch.cuda.synchronize()
+    return stream, dos, call
+
+
+def capture(torch, stream, call):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        call()
+    torch.cuda.synchronize()
+    return graph
+
+
+def test_full_chain_keeps_ends_that_fit():
+    """Under a budget for the ends of whole default segments but not of half ones, a repeated call neither frees
+    nor allocates: it can be captured."""
+    torch = pytest.importorskip("torch")
+    panel, pos, codes = small(seed=8, M=1000, N_=64, B=500)
+    p = N.default_params(num_states=8, ne=20000, flags=N.IMPUTE_FULL_CHAIN | N.IMPUTE_RESELECT)
+    whole, half = ends_bytes(500, 1000, 8, 32), ends_bytes(500, 1000, 8, 16)
+    with Engine(0) as wide:
+        wide.upload_panel(panel); wide.set_map(pos); wide.pbwt_build()
+        _, want, _ = device_call(torch, wide, codes, p)
+        used = wide.memory()[0]
+    with Engine(0, hbm_budget_bytes=used + (whole + half) // 2) as tight:
+        tight.upload_panel(panel); tight.set_map(pos); tight.pbwt_build()
+        stream, dos, call = device_call(torch, tight, codes, p)
+        assert torch.equal(dos, want) and tight.memory()[0] == used  # in parallel
+        graph = capture(torch, stream, call)
+        dos.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(dos, want)
+        del graph
