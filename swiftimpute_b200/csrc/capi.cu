@@ -21,14 +21,14 @@ si_status cuda_fail(si_ctx* ctx, cudaError_t e, const char* what) {
 }
 
 uint64_t reclaimable_bytes(const si_ctx* ctx) {
-    uint64_t b = ctx->bckpt.bytes + ctx->build.bytes;
+    uint64_t b = (ctx->ends_captured ? 0 : ctx->bckpt.bytes) + ctx->build.bytes;
     for (auto& kv : ctx->sel)
         if (kv.second.stale) b += kv.second.pairs.bytes + kv.second.masks.bytes + kv.second.g2.bytes + kv.second.raw.bytes;
     return b;
 }
 
 void reclaim(si_ctx* ctx) {  // cudaFree waits for the kernels that use a buffer
-    dev_free(ctx, ctx->bckpt);
+    if (!ctx->ends_captured) dev_free(ctx, ctx->bckpt);
     dev_free(ctx, ctx->build);
     for (auto it = ctx->sel.begin(); it != ctx->sel.end();) {
         if (!it->second.stale) { ++it; continue; }
@@ -541,7 +541,9 @@ si_status run_device(si_ctx* ctx, const si_impute_params* p, const uint8_t* d_ge
         const size_t need = ends + fb_back_bytes(B, ctx->M, p->num_states, c);
         if (ctx->bckpt.bytes < need) {
             // room beside what an allocation does not reclaim; the ends held now stay where a size does not fit
-            if (ctx->used - reclaimable_bytes(ctx) + need + 255 > ctx->budget) continue;
+            const uint64_t kept = ctx->used - reclaimable_bytes(ctx) - (ctx->ends_captured ? ctx->bckpt.bytes : 0);
+            if (kept + need + 255 > ctx->budget) continue;
+            ctx->ends_captured = false;
             if (dev_alloc(ctx, ctx->bckpt, need) != SI_OK) continue;
         }
         C = c;
@@ -549,6 +551,9 @@ si_status run_device(si_ctx* ctx, const si_impute_params* p, const uint8_t* d_ge
         l.bckpt = (float*)((char*)ctx->bckpt.ptr + ends);
         break;
     }
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    SI_CUDA(ctx, cudaStreamIsCapturing(s, &capturing), "capture status");
+    if (l.bckpt && capturing != cudaStreamCaptureStatusNone) ctx->ends_captured = true;
     if (!l.bckpt) {
         C = whole;
         SI_TRY(dev_reserve(ctx, ctx->ckpt, fb_ckpt_bytes(B, ctx->M, p->num_states, C)));

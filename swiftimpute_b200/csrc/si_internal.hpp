@@ -122,6 +122,7 @@ struct si_ctx {
     si::DeviceBuffer ckpt;           // forward checkpoints (full-chain kernel)
     // Buffers kept between calls while the budget has room and freed for any other allocation (reclaim):
     si::DeviceBuffer bckpt;          // both directions' segment ends (full-chain kernels)
+    bool ends_captured = false;      // bckpt's address is in a captured launch: only a larger call replaces it
     si::DeviceBuffer build;          // start orders and jobs of the index build
     si::DeviceBuffer smasks;         // per-target slot masks [M][B] (target-aware selection)
     // typed-marker kernel scratch and tables

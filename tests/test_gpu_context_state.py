@@ -241,3 +241,32 @@ def test_full_chain_keeps_ends_that_fit():
         torch.cuda.synchronize()
         assert torch.equal(dos, want)
         del graph
+
+
+def test_captured_full_chain_keeps_its_ends():
+    """The ends whose address a captured call holds are no room for other allocations: the graph replays right
+    after the budget has been filled with tables."""
+    torch = pytest.importorskip("torch")
+    panel, pos, codes = small(seed=9, M=1000, N_=64, B=500)
+    p = N.default_params(num_states=8, ne=20000, flags=N.IMPUTE_FULL_CHAIN | N.IMPUTE_RESELECT)
+    ends = ends_bytes(500, 1000, 8, 16)
+    with Engine(0) as wide:
+        wide.upload_panel(panel); wide.set_map(pos); wide.pbwt_build()
+        _, want, _ = device_call(torch, wide, codes, p)
+        used = wide.memory()[0]
+    with Engine(0, hbm_budget_bytes=used + ends + (1 << 20)) as tight:
+        tight.upload_panel(panel); tight.set_map(pos); tight.pbwt_build()
+        stream, dos, call = device_call(torch, tight, codes, p)
+        graph = capture(torch, stream, call)
+        assert tight.memory()[0] >= used + ends  # no longer what another allocation can have
+        for L in range(9, 33):
+            try:
+                tight.select_states(L)
+            except N.SIError as e:
+                assert e.status == ERR_BUDGET
+        dos.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(dos, want)
+        del graph
