@@ -984,15 +984,13 @@ si_status si_pbwt_build(si_ctx* ctx, uint32_t flags) {
     DeviceBuffer scratch, gid, sortbuf;
     si_status st = SI_OK;
     if (scratch_words) st = dev_alloc(ctx, scratch, scratch_words * 4);
+    if (st == SI_OK && S > 1 && !sorted) st = dev_alloc(ctx, gid, (size_t)(S - 1) * N * 4);
+    if (st == SI_OK && S > 1 && !sorted) st = dev_alloc(ctx, sortbuf, (size_t)4 * N * 4);
+    // after the allocations that could reclaim a kept one, perhaps a larger one than this build's
     const size_t job_bytes = (S * sizeof(SweepJob) + 255) & ~size_t(255);
     const size_t build_bytes = job_bytes + (S > 1 ? (sorted ? (size_t)(S - 1) * N * 8 : (size_t)S * N * 4) : 0);
     if (st == SI_OK && ctx->build.bytes < build_bytes) st = dev_alloc(ctx, ctx->build, build_bytes);
-    // the buffer is this call's own until the sweep is through (no allocation below may reclaim it)
-    DeviceBuffer build = ctx->build;
-    ctx->build = DeviceBuffer{};
-    DeviceBuffer jobbuf{build.ptr, 0}, orders{(char*)build.ptr + job_bytes, 0};
-    if (st == SI_OK && S > 1 && !sorted) st = dev_alloc(ctx, gid, (size_t)(S - 1) * N * 4);
-    if (st == SI_OK && S > 1 && !sorted) st = dev_alloc(ctx, sortbuf, (size_t)4 * N * 4);
+    DeviceBuffer jobbuf{ctx->build.ptr, 0}, orders{(char*)ctx->build.ptr + job_bytes, 0};
     cudaError_t e = cudaSuccess;
     if (st == SI_OK) {
         e = cudaMemcpy(jobbuf.ptr, jobs.data(), S * sizeof(SweepJob), cudaMemcpyHostToDevice);
@@ -1022,7 +1020,6 @@ si_status si_pbwt_build(si_ctx* ctx, uint32_t flags) {
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ctx->pbwt_ms, ctx->ev[0], ctx->ev[1]);
     }
     for (DeviceBuffer* b : {&scratch, &gid, &sortbuf}) dev_free(ctx, *b);
-    ctx->build = build;
     if (st != SI_OK) return st;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "PBWT sweep");
     ctx->has_index = true;

@@ -270,3 +270,28 @@ def test_captured_full_chain_keeps_its_ends():
         torch.cuda.synchronize()
         assert torch.equal(dos, want)
         del graph
+
+
+def test_index_build_within_its_budget_after_another_panel():
+    """An index whose build just fits the budget is built after another panel's too, whose larger kept buffer
+    makes room."""
+    M, N_ = 640, 25_000  # 10 segments, swept by groups
+    small_panel, _, _ = synth.make_panel(9600, 1500, 8, seed=10)  # 148 segments, sorted: 1.8 MB of orders
+    rng = np.random.default_rng(11)
+    words = rng.integers(0, 1 << 32, (M, -(-N_ // 32)), dtype=np.uint32) & rng.integers(0, 1 << 32, (M, -(-N_ // 32)), dtype=np.uint32)
+
+    def build(eng):
+        eng.upload_packed(words, N_)
+        eng.pbwt_build(store_index=True)
+        return eng.prefix_rows(M - 1, 1)
+
+    with Engine(0) as wide:
+        want = build(wide)
+        used = wide.memory()[0]
+    # groups' scratch and ranks of nine segments, the sort buffer, ten start orders and the jobs
+    budget = used + 4 * N_ * (4 * 9 + 9 + 4 + 10) + 8192
+    for first in (False, True):
+        with Engine(0, hbm_budget_bytes=budget) as eng:
+            if first:
+                eng.upload_panel(small_panel); eng.pbwt_build()
+            assert np.array_equal(build(eng), want)
