@@ -295,3 +295,36 @@ def test_index_build_within_its_budget_after_another_panel():
             if first:
                 eng.upload_panel(small_panel); eng.pbwt_build()
             assert np.array_equal(build(eng), want)
+
+
+@pytest.mark.parametrize("L,C", [(3, 0), (4, 0), (5, 0), (8, 0), (8, 7), (12, 0), (16, 0), (16, 32), (27, 0), (32, 0), (32, 8)])
+@pytest.mark.parametrize("mode", ["first_gap", "per_gap", "target"])
+def test_full_chain_one_pass(L, C, mode):
+    """The one-pass kernel, which a budget without room for both directions' ends falls back to, and the parallel
+    segments: the same bits. Which of them ran shows in the memory used, where only the one pass' own checkpoints
+    count."""
+    M, B = 1029, 301
+    panel, pos, _ = synth.make_panel(M, 64, 8, seed=L + C, spacing=1000)
+    rng = np.random.default_rng(L + C)
+    pos = np.cumsum(rng.integers(1, 5000, M)).astype(np.uint64)
+    codes = rng.integers(0, 8, (B, M)).astype(np.uint8)  # five cells of eight untyped
+    p = N.default_params(num_states=L, ne=20000, flags=N.IMPUTE_FULL_CHAIN, checkpoint_interval=C,
+                         transition_mode=N.TRANS_PER_GAP if mode == "per_gap" else N.TRANS_MATRIX0,
+                         selection_kind=N.SEL_TARGET if mode == "target" else N.SEL_AUTO)
+
+    def run(eng):
+        eng.upload_panel(panel); eng.set_map(pos); eng.pbwt_build(store_index=True)
+        return eng.impute(codes, p, hap_prob=True)
+
+    lmax = next(x for x in (4, 8, 16, 32) if L <= x)
+    c = C or (16 if lmax == 32 else 32)
+    one = -(-(-(-M // c) - 1) * lmax * B * 4 // 256) * 256
+    assert ends_bytes(B, M, lmax, c) > one + (64 << 10)
+    with Engine(0) as wide:
+        want = run(wide)
+        used = wide.memory()[0]
+    with Engine(0, hbm_budget_bytes=used + one + (64 << 10)) as tight:
+        got = run(tight)
+        assert tight.memory()[0] == used + one
+    for key in want:
+        assert np.array_equal(got[key], want[key]), key
