@@ -224,7 +224,7 @@ pbwt_sweep_kernel(const uint32_t* __restrict__ panel_all, const SweepJob* __rest
 //   sweep    every segment on its own CTA from its start order, writing its
 //            rows (pbwt_sweep_kernel with init_off).
 // The result is bit-identical to one sweep over all markers.
-// Panels whose sort state does not fit a CTA's shared memory (about 20,000
+// Panels whose sort state does not fit a CTA's shared memory (more than 24,811
 // haplotypes) take pbwt_group_kernel for the ranks (a sweep that carries the
 // groups of equal keys) and pbwt_compose_kernel, one segment after the other.
 
@@ -296,7 +296,7 @@ __device__ __forceinline__ void dense_ranks(const uint16_t* ord, uint16_t* rank,
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t E = (N + kSortThreads - 1) / kSortThreads;
     const uint32_t i0 = min(N, t * E), i1 = min(N, i0 + E);
-    uint32_t n = 0, bits = 0;  // E <= 24 at the sizes that fit shared memory
+    uint32_t n = 0, bits = 0;  // E <= 32 (launch_pbwt_orders): 25 at the most haplotypes that fit shared memory
     for (uint32_t i = i0; i < i1; ++i)
         if (i && differs(ord[i - 1], ord[i])) {
             ++n;
@@ -694,6 +694,7 @@ cudaError_t launch_pbwt_orders(const uint32_t* d_panel, const SweepJob* d_jobs, 
                                uint16_t* d_buf, const uint16_t** d_orders, cudaStream_t s) {
     const size_t sm = pbwt_sort_smem_bytes(N, W), words = (size_t)n_jobs * N;
     uint16_t *o = d_buf, *r = o + words, *o2 = r + words, *r2 = o2 + words;
+    if (N > 32 * kSortThreads) return cudaErrorInvalidValue;  // dense_ranks: a bit an element of a thread
     cudaError_t e = allow_smem(pbwt_rank_kernel);
     if (e == cudaSuccess) e = allow_smem(pbwt_double_kernel);
     if (e != cudaSuccess) return e;

@@ -316,3 +316,15 @@ def test_third_cta(engine, L, own):
         a, b = engine.impute(few, p, **out), engine.impute(many, p, **out)
         for key in a:
             assert np.array_equal(a[key][np.arange(B) % 40], b[key]), (key, kw)
+
+
+# the most haplotypes whose index is built by sorting (24,811), one more, and 25 elements a thread (from 24,577)
+@pytest.mark.parametrize("N_", [24576, 24577, 24811, 24812])
+def test_index_largest_sorted(engine, N_):
+    M = 190  # two segments, the second one with a remainder of eight markers
+    rng = np.random.default_rng(N_)
+    panel = (rng.random((M, N_)) < 0.1).astype(np.uint8)
+    panel[:, N_ // 2:] = panel[:, :N_ - N_ // 2]
+    engine.upload_panel(panel)
+    engine.pbwt_build(row_hashes=True)
+    assert np.array_equal(engine.row_hashes(), oracle.pbwt_build_packed(synth.pack_panel(panel), N_)[1])
