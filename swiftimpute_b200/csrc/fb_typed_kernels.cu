@@ -1645,10 +1645,12 @@ __global__ void __launch_bounds__(128, kCtas)
         return;
     }
 
-    // ---- every lane by itself: lanes reach their anchors at different cells. Those at one take it at once,
-    // then all lanes step. (Lanes that waited at an anchor until four of them were there, or none had cells left
-    // in the tile, made the others' wait shorter but left the tile's last cells to few lanes: 9,000 x 6,000, L = 8,
-    // whole calls, a site every 11 markers 2.23 ms against 2.21, every 40 2.35 against 2.22, every 200 4.57 against 3.54.)
+    // ---- every lane by itself: lanes reach their anchors at different cells. A turn of the loop is the anchors of
+    // those at one, or a step of cells for all. (Lanes that waited at an anchor until four of them were there, or none
+    // had cells left in the tile, made the others' wait shorter but left the tile's last cells to few lanes: 9,000 x
+    // 6,000, L = 8, whole calls, a site every 11 markers 2.23 ms against 2.21, every 40 2.35 against 2.22, every 200
+    // 4.57 against 3.54. Anchors and a step in one turn came out of the compiler slower where L is not a power of two:
+    // 9,000 x 3,000, L = 19, every 17: 4.24 ms against 3.46.)
     uint32_t tbase = m & ~31u;
     for (;;) {
         const bool on = live && m < mend;
@@ -1656,15 +1658,16 @@ __global__ void __launch_bounds__(128, kCtas)
         const uint32_t tend = min(tbase + 32, mend), tlo = on ? m - tbase : 32u;
         for (;;) {
             const bool more = on && m < tend, turn = more && m == p1;
-            if (!__any_sync(kAll, more)) break;
-            if (turn) {
-                anchor(tabQS(tb, p1 - p0));
-                p0 = p1;
-                p1 = fr.z;
-                in_tab = p1 - p0 < tb.NT;
-            }
-            __syncwarp();
-            if (more) {  // the next cells of the run, two per step when they pair up
+            const uint32_t turns = __ballot_sync(kAll, turn), steps = __ballot_sync(kAll, more && !turn);
+            if (!(turns | steps)) break;
+            if (turns) {
+                if (turn) {
+                    anchor(tabQS(tb, p1 - p0));
+                    p0 = p1;
+                    p1 = fr.z;
+                    in_tab = p1 - p0 < tb.NT;
+                }
+            } else if (more) {  // the next cells of the run, two per step when they pair up
                 const uint32_t e = min(p1, tend);
                 const bool two = (m & 1u) == 0u && m + 1 < e;
                 float4 qa, qb;
