@@ -244,9 +244,9 @@ __global__ void __launch_bounds__(kStage ? 32 * (1 + kWalkPrep) : 32)
         return;
     }
     const uint32_t s = blockIdx.x * 32 + lane;
-    const bool live = s < B;  // a lane past the batch's end walks too (its staged codes read as missing) and stores nothing
-    const uint8_t* g = geno + (uint64_t)(live ? s : B - 1) * M;
-    SlotMasks* out = smasks + (live ? s : B - 1);
+    if (s >= B) return;  // the barriers below wait for the lanes that stay
+    const uint8_t* g = geno + (uint64_t)s * M;
+    SlotMasks* out = smasks + s;
     uint32_t p = 0;
     for (uint32_t b = 0; b < NB; ++b) {
         if (kStage) __syncthreads();
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kStage ? 32 * (1 + kWalkPrep) : 32)
                 const uint32_t zb = p < N ? zeros[q >> 5] + __popc(~word & ((1u << (p & 31)) - 1u)) : Z;
                 const uint32_t xt = c == 0 ? 0u : c == 2 ? 1u : ((word >> (q & 31)) & 1u);
                 p = xt ? Z + (p - zb) : zb;
-                if (live) out->pad = p;
+                out->pad = p;
                 out += B;
             }
         }
