@@ -1466,12 +1466,13 @@ __global__ void __launch_bounds__(128, kCtas)
         stage_tile(um & ~31u, 0);
         // cells mm and mm + 1 (the second one discarded unless two) into columns c0, c0 + 1, from the run's
         // coefficients and the floor's log at them
-        auto pair_at = [&](uint32_t mm, auto two, const float4 qa, const float4 qb, const float2 ft, uint32_t c0) {
+        auto pair_at = [&](uint32_t mm, auto two, const float4 qa, const float4 qb, auto floor_log, uint32_t c0) {
             const SlotMasks mkA = mrow[c0];
             const SlotMasks mkB = two ? mrow[c0 + 1] : mkA;
             float2 XX = make_float2(qb.x, qb.y), YY = make_float2(qb.z, qb.w);
             // floor e^ft beside X w' + Y; when it dominates (ft > 0) both are scaled by e^-ft. e^-|ft| below the
             // smallest normal number reads 0: it is added to 1 or to Y >= 1e-30, which it would not change.
+            const float2 ft = floor_log();
             const float e0 = ex2_ftz(fabsf(ft.x) * -1.44269504088896341f), e1 = ex2_ftz(fabsf(ft.y) * -1.44269504088896341f);
             const bool big0 = ft.x > 0.f, big1 = ft.y > 0.f;
             const float2 xs = make_float2(big0 ? e0 : 1.f, big1 ? e1 : 1.f);
@@ -1568,9 +1569,11 @@ __global__ void __launch_bounds__(128, kCtas)
             }
         };
         auto pair = [&](uint32_t mm, auto two, const float4* pu, const float4* pd, uint32_t c0) {
-            const float4 gv = pd[1];
-            const float2 ft = __fadd2_rn(__fadd2_rn(FH, make_float2(gv.x, gv.y)), __fadd2_rn(FL, make_float2(gv.z, gv.w)));
-            pair_at(mm, two, *pu, pd[0], ft, c0);
+            const float4 qa = *pu, qb = pd[0], gv = pd[1];
+            auto floor_log = [&] {
+                return __fadd2_rn(__fadd2_rn(FH, make_float2(gv.x, gv.y)), __fadd2_rn(FL, make_float2(gv.z, gv.w)));
+            };
+            pair_at(mm, two, qa, qb, floor_log, c0);
         };
         uint32_t buf = 0;
         for (uint32_t utb = um & ~31u; um < uend; utb += 32, buf ^= 1u) {
@@ -1612,9 +1615,10 @@ __global__ void __launch_bounds__(128, kCtas)
                         const uint32_t j = u1 - um;
                         float4 qa, qb;
                         coeffs(um, qa, qb);
-                        float2 ft = FH;
-                        if (floors) ft = make_float2((float)(fa + tabG(tb, j)), (float)(fa + tabG(tb, j - 1)));
-                        pair_at(um, two, qa, qb, ft, um - utb);
+                        auto floor_log = [&] {
+                            return floors ? make_float2((float)(fa + tabG(tb, j)), (float)(fa + tabG(tb, j - 1))) : FH;
+                        };
+                        pair_at(um, two, qa, qb, floor_log, um - utb);
                         um += two ? 2u : 1u;
                     }
                 }
