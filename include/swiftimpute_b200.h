@@ -114,7 +114,15 @@ si_status si_ctx_create(int device, uint64_t hbm_budget_bytes, si_ctx** out);
 si_status si_ctx_destroy(si_ctx* ctx);
 /* Message of the last failed call on this ctx (never NULL). */
 const char* si_last_error(const si_ctx* ctx);
-/* Replaces Imputer::device_memory_usage (imputer.cpp:1176-1212). */
+/* Replaces Imputer::device_memory_usage (imputer.cpp:1176-1212). used_bytes
+ * leaves out what the ctx keeps allocated between calls only while its budget
+ * has the room, and gives up for any other allocation of the same ctx: the
+ * segment ends of the full-chain kernels (about (8 Lmax + 8) B M / C bytes for B
+ * samples, M markers and segments of C = 16 markers, 8 for L > 16: 0.9 GB for
+ * 4,000 x 50,000 with 8 states), the index build's scratch, and selection tables
+ * of an index since rebuilt. The device memory that the ctx holds is larger by
+ * them after such calls; to another allocator on the device it becomes free with
+ * si_ctx_destroy, and hbm_budget_bytes bounds it. */
 si_status si_ctx_memory(const si_ctx* ctx, uint64_t* used_bytes, uint64_t* budget_bytes);
 
 /* Panel ------------------------------------------------------------------ */
@@ -227,8 +235,8 @@ si_status si_impute_device(si_ctx* ctx, const si_impute_params* p, const uint8_t
  * pool that reserves the free memory and forbids raw allocations beside it),
  * and latency-bound programs that share the device with other streams, where
  * cudaMalloc/cudaFree may synchronise the device. The caller passes device
- * inputs and outputs; the forward checkpoints live in a fixed 16 MiB array
- * inside the library (held by every GPU that loads it, until exit).
+ * inputs and outputs; the checkpoints live in a fixed 16 MiB array inside the
+ * library (held by every GPU that loads it, until exit).
  * It always runs the marker-by-marker (full-chain) recursion, whatever the
  * transition mode; flags other than SI_IMPUTE_FULL_CHAIN are refused. Results
  * agree with si_impute_device within the parity tolerance (1e-4 in dosage),
@@ -238,7 +246,8 @@ si_status si_impute_device(si_ctx* ctx, const si_impute_params* p, const uint8_t
  * 4/8/16/32; more than 16 MiB is refused with SI_ERR_UNSUPPORTED. The ctx must
  * hold the slot and transition tables for these parameters: make one
  * allocating call (si_impute or si_impute_device) with them first, and let it
- * complete. The first call on a ctx is its set-up: it looks up the array's
+ * complete (again after every si_pbwt_build: without it the call answers
+ * SI_ERR_STATE). The first call on a ctx is its set-up: it looks up the array's
  * device address (with lazy module loading, that is also when the driver
  * commits the array's memory); make that call before any stream capture.
  * After a device reset, create a new ctx. Calls share the array, so calls

@@ -140,8 +140,8 @@ __device__ __forceinline__ uint32_t typed_bits(uint4 c) {
 // Anchor counts per segment of kFillSeg markers from a chunk boundary (segment j
 // of a row holds its codes j kFillSeg - a .. (j + 1) kFillSeg - a - 1, the last
 // one the rest): a warp per (sample, segment), its eight 512-byte loads in flight
-// together. Bound by reading the codes: 10,000 x 50,000 in 72 us, 6.9 TB/s of the
-// 6.45 a copy measures (a warp per sample with one load ahead took 163).
+// together. Bound by reading the codes: 4,000 x 50,000 in 34 us, 5.9 TB/s (a copy,
+// which also writes, measures 6.45); a warp per sample with one load ahead took 65.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) anchor_count_kernel(TypedArgs A) {
     const unsigned long long gw = (unsigned long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(kChainThreads, LM <= 16 ? 5 : 3) anchor_chain_
 // 20 for the floor), an anchor about 300. Launch times, one walk for all before
 // -> now: 10,000 x 50,000 (L = 8) 4.06 -> 2.35 ms (writing its 3 GB would take
 // 0.47); 2,003 x 30,011 0.76 -> 0.41; 4,000 x 20,000 (L = 16) 1.27 -> 0.63; 1,500
-// x 6,007 (L = 32, alleles only) 0.22 -> 0.18; one target x 1,644 98 -> 21 us;
+// x 6,007 (L = 32, alleles only) 0.22 -> 0.16; one target x 1,644 98 -> 21 us;
 // 131 x 7,919 with sites of their own (each lane by itself) 1.24 -> 0.22 ms.
 
 // high word of farg' for a uniform run and for a negligible floor

@@ -6,8 +6,8 @@
 // raw allocations beside it), and latency-bound callers that share the device
 // with other streams (cudaMalloc and cudaFree may synchronise the device, which
 // stalls the other streams' work). The caller allocates inputs and outputs;
-// the forward checkpoints, the only scratch this path needs, live in a fixed
-// array compiled into the library.
+// the checkpoints, the only scratch this path needs, live in a fixed array
+// compiled into the library.
 //
 // The array below is a file-scope __device__ variable: every GPU that loads
 // this library holds kNoAllocScratchBytes of it until the process exits. In
@@ -27,7 +27,7 @@
 namespace si {
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = 16u << 20;  // 16 MiB of forward checkpoints
+constexpr size_t kNoAllocScratchBytes = 16u << 20;  // 16 MiB of checkpoints
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
